@@ -441,17 +441,6 @@ struct SegCountF {
         return len > thr ? (uint32_t)((len + seg - 1) / seg) : 0u;
     }
 };
-// 1 where a run of non-hub rows starts
-struct RunStartF {
-    const int64_t *ptr;
-    int64_t thr;
-    __device__ uint32_t operator()(int64_t r) const
-    {
-        const bool hub = ptr[r + 1] - ptr[r] > thr;
-        return !hub && (r == 0 || ptr[r] - ptr[r - 1] > thr);
-    }
-};
-
 __global__ void hub_segments_kernel(const int64_t *ptr, int64_t N, int64_t thr, int64_t seg, const uint32_t *hubpos,
                                     const uint32_t *segoff, int64_t nhub, int64_t nseg, int32_t *hub_row,
                                     int64_t *hub_seg, int32_t *seg_row, int64_t *seg_beg)
@@ -473,47 +462,151 @@ __global__ void hub_segments_kernel(const int64_t *ptr, int64_t N, int64_t thr, 
         hub_seg[nhub] = nseg;
 }
 
-// The host's greedy packing of rows into tasks (a row costs its entries plus
-// 2; a task closes once its cost reaches te; hub rows close a task and belong
-// to none), run independently on every run of non-hub rows, which is exactly
-// where the greedy state is reset.  Pass 1 (rb == nullptr) counts each run's
-// tasks into cnt; pass 2 writes them from off[run] on.
-__global__ void run_tasks_kernel(const int64_t *ptr, int64_t N, int64_t thr, int64_t te, const uint32_t *runpos,
-                                 uint32_t *cnt, const uint32_t *off, int32_t *rb, int32_t *re)
+// ---------------------------------------------------------------------------
+// The host's greedy packing of rows into tasks: a row costs its entries plus 2,
+// a task closes once its cost reaches te, a hub row closes the open task and
+// belongs to none.  Where a task that starts at row s ends depends on s alone,
+// so the packing is the chain s -> next(s) from row 0 (a hub row steps to the
+// row after it), and the tasks are the non-hub rows on it.  next() is computed
+// for every row at once (binary search: a task has at most ceil(te / 2) rows)
+// and the chain is followed block by block: kTaskBlock rows are jumped at a
+// time through exit[] (the first row on the chain from s that lies past s's
+// block), kTaskSuper blocks at a time through exit2[], so the serial part is
+// one load per kTaskBlock * kTaskSuper rows.  Bound by that chain and by launch
+// latency.  Following the greedy row by row, one thread per run of non-hub rows,
+// took 18.1 ms on an R-MAT graph of 1 M rows (14 M entries; its runs are up to
+// tens of thousands of rows long); these kernels take 0.14 ms together.
+// ---------------------------------------------------------------------------
+constexpr int kTaskItems = 8;                        // rows per thread
+constexpr int kTaskBlock = kThreads * kTaskItems;    // rows jumped by exit[]
+constexpr int kTaskSuper = 16;                       // blocks jumped by exit2[]
+constexpr int64_t kSuperRows = (int64_t)kTaskBlock * kTaskSuper;
+
+__global__ void task_next_kernel(const int64_t *ptr, int64_t N, int64_t thr, int64_t te, const uint32_t *hubpos,
+                                 int32_t *next)
 {
-    for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < N; a += (int64_t)gridDim.x * blockDim.x) {
-        const bool hub_a = ptr[a + 1] - ptr[a] > thr;
-        if (hub_a || (a > 0 && !(ptr[a] - ptr[a - 1] > thr)))
-            continue;  // not the first row of a run
-        const uint32_t run = runpos[a];
-        uint32_t t = rb ? off[run] : 0u, k = 0;
-        int64_t start = -1, cost = 0, r = a;
-        for (; r < N; r++) {
-            const int64_t len = ptr[r + 1] - ptr[r];
-            if (len > thr)
-                break;
-            if (start < 0)
-                start = r;
-            cost += len + 2;
-            if (cost >= te) {
-                if (rb) {
-                    rb[t + k] = (int32_t)start;
-                    re[t + k] = (int32_t)(r + 1);
-                }
-                k++;
-                start = -1;
-                cost = 0;
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N; s += (int64_t)gridDim.x * blockDim.x) {
+        // the first e in (s, hi] at which the task [s, e) closes: its cost has
+        // reached te, or row e - 1 is a hub (then it closes before that row)
+        const int64_t b = ptr[s];
+        const uint32_t h = hubpos[s];
+        int64_t lo = s + 1, hi = min(N, s + (te + 1) / 2);
+        while (lo < hi) {
+            const int64_t e = (lo + hi) >> 1;
+            const int64_t pe = ptr[e];
+            if (pe - b + 2 * (e - s) >= te || hubpos[e - 1] + (pe - ptr[e - 1] > thr ? 1u : 0u) > h)
+                hi = e;
+            else
+                lo = e + 1;
+        }
+        next[s] = (int32_t)lo;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) task_exit_kernel(const int32_t *next, int64_t N, int32_t *exit)
+{
+    __shared__ int32_t a[kTaskBlock];
+    const int64_t base = (int64_t)blockIdx.x * kTaskBlock, end = min(N, base + kTaskBlock);
+    for (int j = threadIdx.x; base + j < end; j += kThreads)
+        a[j] = next[base + j];
+    __syncthreads();
+    // pointer doubling: after round i, a[j] is 2^i steps on or past the block
+    for (int len = 1; len < kTaskBlock; len <<= 1) {
+        int32_t v[kTaskItems];
+        int more = 0;
+#pragma unroll
+        for (int q = 0; q < kTaskItems; q++) {
+            const int j = threadIdx.x + q * kThreads;
+            v[q] = base + j < end ? a[j] : (int32_t)end;
+            if (v[q] < end) {
+                v[q] = a[v[q] - base];
+                more = 1;
             }
         }
-        if (start >= 0) {
-            if (rb) {
-                rb[t + k] = (int32_t)start;
-                re[t + k] = (int32_t)r;
-            }
-            k++;
+        more = __syncthreads_or(more);
+#pragma unroll
+        for (int q = 0; q < kTaskItems; q++)
+            if (base + threadIdx.x + q * kThreads < end)
+                a[threadIdx.x + q * kThreads] = v[q];
+        __syncthreads();
+        if (!more)
+            break;
+    }
+    for (int j = threadIdx.x; base + j < end; j += kThreads)
+        exit[base + j] = a[j];
+}
+
+// exit2[i], i = sb * kTaskBlock + j: from row j of superblock sb's first block
+// to the first row on the chain past the superblock.
+__global__ void task_exit2_kernel(const int32_t *exit, int64_t N, int64_t nsuper, int32_t *exit2)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nsuper * kTaskBlock;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t sb = i / kTaskBlock, end = min(N, (sb + 1) * kSuperRows);
+        int64_t s = sb * kSuperRows + i % kTaskBlock;
+        while (s < end)
+            s = exit[s];
+        exit2[i] = (int32_t)min(s, N);
+    }
+}
+
+// One block: entry[b] = the first row of block b on the chain, or -1.
+__global__ void __launch_bounds__(kThreads) task_walk_kernel(const int32_t *exit, const int32_t *exit2, int64_t N,
+                                                             int64_t nsuper, int32_t *super_entry, int32_t *entry)
+{
+    if (threadIdx.x == 0)
+        for (int64_t s = 0, last = -1; s < N;) {
+            const int64_t sb = s / kSuperRows;
+            if (sb != last)
+                super_entry[sb] = (int32_t)s;
+            last = sb;
+            const int64_t j = s - sb * kSuperRows;
+            s = j < kTaskBlock ? exit2[sb * kTaskBlock + j] : exit[s];
         }
-        if (!rb)
-            cnt[run] = k;
+    __syncthreads();
+    for (int64_t sb = threadIdx.x; sb < nsuper; sb += kThreads) {
+        const int64_t end = min(N, (sb + 1) * kSuperRows);
+        int64_t s = super_entry[sb];
+        while (s >= 0 && s < end) {
+            entry[s / kTaskBlock] = (int32_t)s;
+            s = exit[s];
+        }
+    }
+}
+
+// start[r] = 1 where a task starts: the non-hub rows on the chain.
+__global__ void __launch_bounds__(kThreads) task_starts_kernel(const int64_t *ptr, const int32_t *next, int64_t N,
+                                                               int64_t thr, const int32_t *entry, uint32_t *start)
+{
+    __shared__ int32_t a[kTaskBlock];
+    __shared__ unsigned char on[kTaskBlock];
+    const int64_t base = (int64_t)blockIdx.x * kTaskBlock, end = min(N, base + kTaskBlock);
+    for (int j = threadIdx.x; base + j < end; j += kThreads) {
+        a[j] = next[base + j];
+        on[j] = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int64_t first = entry[blockIdx.x];
+        for (int64_t s = first; s >= 0 && s < end; s = a[s - base])
+            on[s - base] = 1;
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; base + j < end; j += kThreads)
+        start[base + j] = on[j] && ptr[base + j + 1] - ptr[base + j] <= thr;
+}
+
+// Task pos[r] of every row r with start[r]: rows [r, next(r)), without the hub
+// row that closed it.
+__global__ void task_write_kernel(const int64_t *ptr, const int32_t *next, int64_t N, int64_t thr,
+                                  const uint32_t *start, const uint32_t *pos, int32_t *rb, int32_t *re)
+{
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
+        if (!start[r])
+            continue;
+        const int64_t e = next[r];
+        rb[pos[r]] = (int32_t)r;
+        re[pos[r]] = (int32_t)(ptr[e] - ptr[e - 1] > thr ? e - 1 : e);
     }
 }
 
@@ -932,10 +1025,10 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
         const size_t scan_blocks = (size_t)((std::max<int64_t>(std::max<int64_t>(ntiles * kBins, nnz), N + 1) +
                                              kScanTile - 1) / kScanTile) + 1;
         // sort keys and ids (x2), digit counts, unique positions, values and
-        // columns, row pointers, hub / segment / run positions, run task
-        // counts and offsets, small values, the scans' block sums
+        // columns, row pointers, hub and segment positions, the task packing's
+        // row arrays, small values, the scans' block sums
         const size_t bytes = 2 * (8 * n + a) + 2 * (4 * n + a) + (4 * (size_t)ntiles * kBins + a) + 3 * (4 * n + a) +
-                             (8 * rows + a) + 5 * (4 * rows + a) + 4 * a + 24 * (4 * scan_blocks + a);
+                             (8 * rows + a) + 7 * (4 * (rows + kTaskBlock) + a) + 6 * a + 24 * (4 * scan_blocks + a);
         COLA_TRY(sc.reserve(bytes));
     }
     if (nnz > 0)
@@ -979,23 +1072,33 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
         COLA_CUDA(cudaMemsetAsync(rv_ptr, 0, ((size_t)N + 1) * 8, st));
     }
     COLA_CUDA(cudaGetLastError());
-    // hub rows and their segments; runs of non-hub rows and their tasks
-    uint32_t nhub = 0, nseg = 0, nrun = 0, ntask = 0;
-    uint32_t *hubpos = nullptr, *segoff = nullptr, *runpos = nullptr, *cnt = nullptr, *toff = nullptr;
+    // hub rows and their segments; the tasks of the other rows
+    uint32_t nhub = 0, nseg = 0, ntask = 0;
+    uint32_t *hubpos = nullptr, *segoff = nullptr, *tstart = nullptr, *tpos = nullptr;
+    int32_t *tnext = nullptr, *texit = nullptr, *texit2 = nullptr, *tentry = nullptr, *tsuper = nullptr;
+    const int64_t ntb = ((int64_t)N + kTaskBlock - 1) / kTaskBlock, nsuper = (ntb + kTaskSuper - 1) / kTaskSuper;
     COLA_TRY(sc.get(hubpos, N));
     COLA_TRY(sc.get(segoff, N));
-    COLA_TRY(sc.get(runpos, N));
+    COLA_TRY(sc.get(tnext, N));
+    COLA_TRY(sc.get(texit, N));
+    COLA_TRY(sc.get(tstart, N));
+    COLA_TRY(sc.get(tpos, N));
+    COLA_TRY(sc.get(texit2, nsuper * kTaskBlock));
+    COLA_TRY(sc.get(tentry, ntb));
+    COLA_TRY(sc.get(tsuper, nsuper));
     COLA_TRY(exclusive_scan(HubF{rv_ptr, thr}, N, hubpos, d_total, &nhub, sc));
     COLA_TRY(exclusive_scan(SegCountF{rv_ptr, thr, seg}, N, segoff, d_total, &nseg, sc));
-    COLA_TRY(exclusive_scan(RunStartF{rv_ptr, thr}, N, runpos, d_total, &nrun, sc));
-    COLA_TRY(sc.get(cnt, nrun));
-    COLA_TRY(sc.get(toff, nrun));
-    if (nrun > 0) {
-        run_tasks_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(rv_ptr, N, thr, te, runpos, cnt, nullptr, nullptr,
-                                                                nullptr);
-        t_launches++;
+    if (N > 0) {
+        task_next_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(rv_ptr, N, thr, te, hubpos, tnext);
+        task_exit_kernel<<<(unsigned)ntb, kThreads, 0, st>>>(tnext, N, texit);
+        task_exit2_kernel<<<grid_stride_blocks(nsuper * kTaskBlock), 256, 0, st>>>(texit, N, nsuper, texit2);
+        COLA_CUDA(cudaMemsetAsync(tsuper, 0xff, (size_t)nsuper * 4, st));
+        COLA_CUDA(cudaMemsetAsync(tentry, 0xff, (size_t)ntb * 4, st));
+        task_walk_kernel<<<1, kThreads, 0, st>>>(texit, texit2, N, nsuper, tsuper, tentry);
+        task_starts_kernel<<<(unsigned)ntb, kThreads, 0, st>>>(rv_ptr, tnext, N, thr, tentry, tstart);
+        t_launches += 5;
         COLA_CUDA(cudaGetLastError());
-        COLA_TRY(exclusive_scan(ArrayF{cnt}, nrun, toff, d_total, &ntask, sc));
+        COLA_TRY(exclusive_scan(ArrayF{tstart}, N, tpos, d_total, &ntask, sc));
     }
     // nnz in the partitions' local blocks
     unsigned long long *d_local = nullptr, h_local = 0;
@@ -1037,12 +1140,10 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
             reinterpret_cast<int64_t *>(base + o_hseg), reinterpret_cast<int32_t *>(base + o_srow),
             reinterpret_cast<int64_t *>(base + o_sbeg));
         t_launches++;
-        if (nrun > 0) {
-            run_tasks_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(ptr_final, N, thr, te, runpos, nullptr, toff,
-                                                                    reinterpret_cast<int32_t *>(base + o_trb),
-                                                                    reinterpret_cast<int32_t *>(base + o_tre));
-            t_launches++;
-        }
+        task_write_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(ptr_final, tnext, N, thr, tstart, tpos,
+                                                                 reinterpret_cast<int32_t *>(base + o_trb),
+                                                                 reinterpret_cast<int32_t *>(base + o_tre));
+        t_launches++;
         COLA_CUDA(cudaGetLastError());
     } else {
         const int64_t zero = 0;
