@@ -20,8 +20,8 @@
 #include "tune_cache.h"
 
 using cola::dev::BatchGraph;
-static_assert(cola::kBatchQueueBytes >= (cola::dev::kMaxItemQueues + 1) * sizeof(unsigned int),
-              "the batch counters must hold the kernel's counters");
+static_assert(cola::kBatchQueueBytes >= 2 * cola::kBatchGroups * sizeof(unsigned int),
+              "an item counter and a count of finished warps per group");
 
 struct cola_batch {
     int device = 0;
@@ -33,6 +33,7 @@ struct cola_batch {
     std::vector<BatchGraph> h_desc;  // graphs that run in the batched launch
     BatchGraph *d_desc = nullptr;
     size_t d_desc_bytes = 0;
+    cola::BatchLaunch launch = {};  // groups and totals of h_desc
     int64_t total_items = 0, total_hub = 0;
     struct Solo {  // graphs that run through cola_spmm (scalar path or K > 32 vectors)
         int g;
@@ -74,53 +75,96 @@ static void batch_release(cola_batch *b)
     delete b;
 }
 
-template <typename TR, typename TY, int UNROLL, int MINB>
-static cola_status launch_batch_t(const BatchLaunch &L, cudaStream_t st)
+template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB>
+static cola_status launch_group_t(const BatchLaunch &L, int i, cudaStream_t st)
 {
-    const bool dyn = L.queue && L.total_items < INT32_MAX;
-    auto fn = dyn ? dev::batch_rowblock_kernel<TR, TY, UNROLL, MINB, true>
-                  : dev::batch_rowblock_kernel<TR, TY, UNROLL, MINB, false>;
-    int64_t gx = grid_for((const void *)fn, L.total_items);
+    const BatchGroup &G = L.group[i];
+    const bool dyn = L.queue != nullptr;
+    auto fn = dyn ? dev::batch_rowblock_kernel<TR, TY, LG, NV, UNROLL, MINB, true>
+                  : dev::batch_rowblock_kernel<TR, TY, LG, NV, UNROLL, MINB, false>;
+    int64_t gx = grid_for((const void *)fn, G.items);
     gx = std::max<int64_t>(1, gx * L.grid_pct / 100);
     t_launches++;
-    fn<<<(unsigned)gx, dev::kThreads, 0, st>>>(L.desc, L.ngraphs, L.total_items, L.accumulate,
-                                               dyn ? L.queue : nullptr);
-    COLA_CUDA(cudaGetLastError());
+    // groups write different outputs: a group may start while the one before it
+    // drains (it waits for that one at its end)
+    COLA_CUDA(launch_kernel(fn, (unsigned)gx, 1, i > 0, st, L.desc + G.first, G.count, (unsigned int)G.items,
+                            L.accumulate, dyn ? L.queue + i : nullptr, dyn ? L.queue + kBatchGroups + i : nullptr));
     return COLA_SUCCESS;
 }
 
+// Loads in flight per lane group and resident blocks are those of the
+// single-graph launch for the width; the batch's own parameters apply to full
+// warps (lane width 32), where every choice sums in the same order.
 template <typename TR, typename TY>
-static cola_status launch_batch_u(const BatchLaunch &L, cudaStream_t st)
+static cola_status launch_group(const BatchLaunch &L, int i, cudaStream_t st)
 {
-    if (L.blocks_per_sm == 3)
-        return L.unroll == 2 ? launch_batch_t<TR, TY, 2, 3>(L, st) : launch_batch_t<TR, TY, 4, 3>(L, st);
-    return L.unroll == 2 ? launch_batch_t<TR, TY, 2, 4>(L, st) : launch_batch_t<TR, TY, 4, 4>(L, st);
+    switch (L.group[i].lg) {
+    case 1:
+        return launch_group_t<TR, TY, 1, 1, 1, 4>(L, i, st);
+    case 2:
+        return launch_group_t<TR, TY, 2, 1, 2, 4>(L, i, st);
+    case 4:
+        return launch_group_t<TR, TY, 4, 1, 4, 4>(L, i, st);
+    case 8:
+        return launch_group_t<TR, TY, 8, 1, 4, 4>(L, i, st);
+    case 16:
+        return launch_group_t<TR, TY, 16, 1, 4, 4>(L, i, st);
+    case 32:
+        if (L.blocks_per_sm == 3)
+            return L.unroll == 2 ? launch_group_t<TR, TY, 32, 1, 2, 3>(L, i, st)
+                                 : launch_group_t<TR, TY, 32, 1, 4, 3>(L, i, st);
+        return L.unroll == 2 ? launch_group_t<TR, TY, 32, 1, 2, 4>(L, i, st)
+                             : launch_group_t<TR, TY, 32, 1, 4, 4>(L, i, st);
+    default:
+        return L.unroll == 2 ? launch_group_t<TR, TY, 32, 2, 2, 4>(L, i, st)
+                             : launch_group_t<TR, TY, 32, 2, 4, 3>(L, i, st);
+    }
 }
 
 cola_status launch_batch(const BatchLaunch &L, cudaStream_t st)
 {
     using BF = __nv_bfloat16;
-    if (L.total_items > 0) {
-        cola_status s;
+    for (int i = 0; i < L.ngroups; i++) {
         if (L.xdt == COLA_FLOAT32)
-            s = L.ydt == COLA_FLOAT32 ? launch_batch_u<dev::VecTraits<float>, float>(L, st)
-                                      : launch_batch_u<dev::VecTraits<float>, BF>(L, st);
+            COLA_TRY((L.ydt == COLA_FLOAT32 ? launch_group<dev::VecTraits<float>, float>(L, i, st)
+                                            : launch_group<dev::VecTraits<float>, BF>(L, i, st)));
         else
-            s = L.ydt == COLA_FLOAT32 ? launch_batch_u<dev::VecTraits<BF>, float>(L, st)
-                                      : launch_batch_u<dev::VecTraits<BF>, BF>(L, st);
-        COLA_TRY(s);
+            COLA_TRY((L.ydt == COLA_FLOAT32 ? launch_group<dev::VecTraits<BF>, float>(L, i, st)
+                                            : launch_group<dev::VecTraits<BF>, BF>(L, i, st)));
     }
     if (L.total_hub > 0) {
-        const int64_t blocks = std::min<int64_t>((L.total_hub + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock,
-                                                 (int64_t)sm_count() * 16);
+        const int lanes = dev::hub_lanes(L.kmax);
+        const unsigned blocks = hub_blocks(L.total_hub, lanes);
         t_launches++;
         if (L.ydt == COLA_FLOAT32)
-            dev::batch_hub_combine_kernel<float, 4><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                L.desc, L.ngraphs, L.total_hub, L.accumulate);
+            COLA_CUDA(launch_kernel(dev::batch_hub_combine_kernel<float>, blocks, 1, true, st, L.desc, L.ngraphs,
+                                    L.total_hub, lanes, L.accumulate));
         else
-            dev::batch_hub_combine_kernel<BF, 4><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                L.desc, L.ngraphs, L.total_hub, L.accumulate);
-        COLA_CUDA(cudaGetLastError());
+            COLA_CUDA(launch_kernel(dev::batch_hub_combine_kernel<BF>, blocks, 1, true, st, L.desc, L.ngraphs,
+                                    L.total_hub, lanes, L.accumulate));
+    }
+    return COLA_SUCCESS;
+}
+
+cola_status build_groups(BatchGraph *d, int n, BatchLaunch &L)
+{
+    std::stable_sort(d, d + n, [](const BatchGraph &a, const BatchGraph &b) { return a.lg < b.lg; });
+    L.ngroups = 0;
+    L.ngraphs = n;
+    L.total_hub = 0;
+    L.kmax = 0;
+    for (int i = 0; i < n; i++) {
+        if (i == 0 || d[i].lg != d[i - 1].lg)
+            L.group[L.ngroups++] = {d[i].lg, i, 0, 0};
+        BatchGroup &G = L.group[L.ngroups - 1];
+        G.count++;
+        d[i].item0 = G.items;
+        G.items += d[i].ba.nitem;
+        COLA_REQUIRE(G.items < INT32_MAX, COLA_ERROR_UNSUPPORTED, "batch: %lld work items (2^31 at most)",
+                     (long long)G.items);
+        d[i].hub0 = L.total_hub;
+        L.total_hub += d[i].nhub * dev::hub_tiles(d[i].K);
+        L.kmax = std::max(L.kmax, (int)d[i].K);
     }
     return COLA_SUCCESS;
 }
@@ -129,25 +173,15 @@ void fill_batch_graph(BatchGraph &d, const cola_graph *g, const void *X, int64_t
                       cola_dtype xdt, float *ws)
 {
     std::memset(&d, 0, sizeof d);
-    d.ba.rowptr = g->rv_ptr;
-    d.ba.col = g->rv_col;
-    d.ba.val = g->rv_val;
-    d.ba.task_rb = g->task_rb;
-    d.ba.task_re = g->task_re;
-    d.ba.ntask = g->ntask;
-    d.ba.seg_row = g->seg_row;
-    d.ba.seg_beg = g->seg_beg;
-    d.ba.nseg = g->nseg;
-    d.ba.seg_len = g->hub_segment;
-    d.ba.queue = nullptr;  // the batch kernel assigns items statically
-    d.ba.ws = ws;
-    d.ba.ld_ws = K;
+    d.ba = block_args(g, ws, K);
+    d.ba.queue = nullptr;  // the launch has its own counters
     d.X = X;
     d.ldx = ldx;
     d.Y = Y;
     d.ldy = ldy;
     d.K = K;
-    d.lg = dev::batch_lane_width(K, xdt == COLA_FLOAT32 ? 4 : 8);
+    const int E = xdt == COLA_FLOAT32 ? 4 : 8;
+    d.lg = K > 32 * E ? 64 : row_lanes(K, E);
     d.hub_row = g->hub_row;
     d.hub_seg = g->hub_seg;
     d.nhub = g->nhub;
@@ -160,11 +194,8 @@ static cola_status batch_run(cola_batch *b, const cola_spmm_opts *opts, cudaStre
     COLA_REQUIRE(!(accumulate && b->ydt != COLA_FLOAT32), COLA_ERROR_UNSUPPORTED,
                  "cola_batch_run: accumulate needs FP32 outputs");
     const int64_t before = t_launches;
-    BatchLaunch L;
+    BatchLaunch L = b->launch;
     L.desc = b->d_desc;
-    L.ngraphs = (int)b->h_desc.size();
-    L.total_items = b->total_items;
-    L.total_hub = b->total_hub;
     L.xdt = b->xdt;
     L.ydt = b->ydt;
     L.unroll = b->unroll;
@@ -311,24 +342,26 @@ cola_status cola_batch_bind(cola_batch *b, const void *const *X, const int64_t *
                      (long long)ldx[i], (long long)ldy[i]);
         if (g->N == 0)
             continue;
-        COLA_REQUIRE(g->nseg + g->ntask < INT32_MAX, COLA_ERROR_UNSUPPORTED,
-                     "cola_batch_bind: graph %zu has %lld work items (2^31 at most)", i, (long long)(g->nseg + g->ntask));
         if (g->nseg > 0)
             COLA_TRY(ensure(reinterpret_cast<void *&>(g->ws_hub), g->ws_hub_bytes,
                             (size_t)g->nseg * K[i] * sizeof(float)));
+        // a graph that is in the batch twice has one hub workspace: its second
+        // product runs after the batch
+        bool again = false;
+        for (size_t j = 0; j < i && g->nseg > 0 && !again; j++)
+            again = b->graphs[j] == g;
         const bool vec = vec_ok_rows(xdt, X[i], ldx[i], ydt, Y[i], ldy[i], K[i]) && aligned16(g->ws_hub);
-        if (!vec) {
+        if (!vec || again) {
             b->solo.push_back({(int)i, X[i], ldx[i], Y[i], ldy[i], K[i]});
             continue;
         }
         BatchGraph d;
         fill_batch_graph(d, g, X[i], ldx[i], Y[i], ldy[i], K[i], xdt, g->ws_hub);
-        d.item0 = b->total_items;
-        d.hub0 = b->total_hub;
         b->total_items += g->nseg + g->ntask;
-        b->total_hub += g->nhub * ((K[i] + 127) / 128);
         b->h_desc.push_back(d);
     }
+    COLA_TRY(build_groups(b->h_desc.data(), (int)b->h_desc.size(), b->launch));
+    b->total_hub = b->launch.total_hub;
     const size_t qoff = batch_queue_offset(b->h_desc.size() * sizeof(BatchGraph));
     const size_t need = qoff + kBatchQueueBytes;
     void *p = b->d_desc;

@@ -31,6 +31,37 @@ int64_t grid_for(const void *fn, int64_t items);
 inline bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // Vector path of the row-major schedule for these operands.
 bool vec_ok_rows(cola_dtype xdt, const void *X, int64_t ldx, cola_dtype ydt, const void *Y, int64_t ldy, int K);
+// Lanes that cover a row of K features in 16-byte vectors of E, at most 32.
+inline int row_lanes(int K, int E)
+{
+    int lg = 1;
+    while (lg < 32 && lg * E < K)
+        lg <<= 1;
+    return lg;
+}
+// A launch of dev::kThreads threads a block; `overlap`: its blocks may start
+// before the kernel launched before it on the stream has ended (it says itself
+// where it waits, griddepcontrol.wait).
+template <typename... P, typename... A>
+cudaError_t launch_kernel(void (*fn)(P...), unsigned gx, unsigned gy, bool overlap, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gx, gy);
+    cfg.blockDim = dim3(dev::kThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+// Blocks of the hub combine (its items stride over the blocks).
+inline unsigned hub_blocks(int64_t items, int lanes)
+{
+    const int64_t per = dev::kThreads / lanes, need = (items + per - 1) / per, most = (int64_t)sm_count() * 16;
+    return (unsigned)(need < 1 ? 1 : need < most ? need : most);
+}
 // Grow a device allocation to at least `need` bytes (contents not kept).
 cola_status ensure(void *&p, size_t &have, size_t need);
 
@@ -81,14 +112,15 @@ struct cola_graph {
     // row-major view (ROWS schedule): merged local + transposed remote entries
     bool has_rows = false;
     const int64_t *rv_ptr = nullptr;  // N+1
-    const int32_t *rv_col = nullptr;
+    const int32_t *rv_col = nullptr;  // dev::kRowEnd on each row's last entry
     const float *rv_val = nullptr;
     const int32_t *seg_row = nullptr;
     const int64_t *seg_beg = nullptr;
     const int32_t *hub_row = nullptr;
     const int64_t *hub_seg = nullptr;
-    const int32_t *task_rb = nullptr, *task_re = nullptr;
-    int64_t nseg = 0, nhub = 0, ntask = 0;
+    const void *items = nullptr;  // dev::WorkItem: segments, then tasks
+    const int32_t *nz_row = nullptr, *empty_row = nullptr;
+    int64_t nseg = 0, nhub = 0, ntask = 0, nempty = 0;
     int32_t hub_threshold = 256, hub_segment = 256, task_entries = 128;
     float *ws_hub = nullptr;  // nseg x K partials
     // dev::kMaxItemQueues + 1 work-item counters of the row-major schedule,

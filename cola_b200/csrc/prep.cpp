@@ -527,6 +527,29 @@ cola_status validate_partition(const cola_partition_set &s, const PartHost &P)
     return COLA_SUCCESS;
 }
 
+void build_row_items(RowView &rv, int64_t hub_segment, int32_t row_end_mark, int32_t pad, RowItems &ri)
+{
+    const int64_t N = (int64_t)rv.ptr.size() - 1;
+    std::vector<int32_t> nzpos((size_t)N + 1, 0);  // rows with entries before row r
+    for (int64_t r = 0; r < N; r++) {
+        const int64_t e = rv.ptr[(size_t)r + 1];
+        const bool some = e > rv.ptr[(size_t)r];
+        nzpos[(size_t)r + 1] = nzpos[(size_t)r] + (some ? 1 : 0);
+        (some ? ri.nz_row : ri.empty_row).push_back((int32_t)r);
+        if (some)
+            rv.col[(size_t)e - 1] |= row_end_mark;
+    }
+    ri.nz_row.resize(ri.nz_row.size() + (size_t)pad, 0);
+    for (size_t s = 0; s < rv.seg_row.size(); s++) {
+        const int64_t e = rv.ptr[(size_t)rv.seg_row[s] + 1];
+        ri.item.push_back({rv.seg_beg[s], (int32_t)std::min<int64_t>(hub_segment, e - rv.seg_beg[s]), 0});
+    }
+    for (size_t t = 0; t < rv.task_rb.size(); t++) {
+        const int64_t b = rv.ptr[(size_t)rv.task_rb[t]];
+        ri.item.push_back({b, (int32_t)(rv.ptr[(size_t)rv.task_re[t]] - b), nzpos[(size_t)rv.task_rb[t]]});
+    }
+}
+
 cola_status build_row_view(const cola_partition_set &s, int64_t hub_threshold, int64_t hub_segment,
                            int64_t task_entries, RowView &rv)
 {

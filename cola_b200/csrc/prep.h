@@ -81,6 +81,19 @@ struct RowView {
 cola_status build_row_view(const cola_partition_set &s, int64_t hub_threshold, int64_t hub_segment,
                            int64_t task_entries, RowView &rv);
 
+// What the device's row view adds: the work items (segments, then tasks), the
+// lists of rows with and without entries (the first padded by `pad`), and the
+// mark on each row's last column.
+struct RowItem {
+    int64_t beg;
+    int32_t n, out;
+};
+struct RowItems {
+    std::vector<RowItem> item;
+    std::vector<int32_t> nz_row, empty_row;
+};
+void build_row_items(RowView &rv, int64_t hub_segment, int32_t row_end_mark, int32_t pad, RowItems &ri);
+
 }  // namespace cola
 
 struct cola_partition_set {

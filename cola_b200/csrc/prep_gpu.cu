@@ -32,6 +32,7 @@
 #include "common.h"
 #include "graph.h"
 #include "prep.h"
+#include "spmm_rows.cuh"
 
 namespace cola {
 namespace pg {
@@ -431,6 +432,11 @@ struct HubF {
     int64_t thr;
     __device__ uint32_t operator()(int64_t r) const { return ptr[r + 1] - ptr[r] > thr; }
 };
+// 1 per row with entries
+struct SomeF {
+    const int64_t *ptr;
+    __device__ uint32_t operator()(int64_t r) const { return ptr[r + 1] > ptr[r]; }
+};
 // segments of row r: ceil(len / seg) for a hub row, else 0
 struct SegCountF {
     const int64_t *ptr;
@@ -441,12 +447,21 @@ struct SegCountF {
         return len > thr ? (uint32_t)((len + seg - 1) / seg) : 0u;
     }
 };
-__global__ void hub_segments_kernel(const int64_t *ptr, int64_t N, int64_t thr, int64_t seg, const uint32_t *hubpos,
-                                    const uint32_t *segoff, int64_t nhub, int64_t nseg, int32_t *hub_row,
-                                    int64_t *hub_seg, int32_t *seg_row, int64_t *seg_beg)
+// Per row: its place in the list of rows with or without entries, the mark on
+// its last column, and a hub's segments with their work items.
+__global__ void rows_kernel(const int64_t *ptr, int64_t N, int64_t thr, int64_t seg, const uint32_t *hubpos,
+                            const uint32_t *segoff, const uint32_t *nzpos, int64_t nhub, int64_t nseg,
+                            int32_t *hub_row, int64_t *hub_seg, int32_t *seg_row, int64_t *seg_beg,
+                            dev::WorkItem *item, int32_t *nz_row, int32_t *empty_row, int32_t *rv_col)
 {
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = ptr[r], e = ptr[r + 1];
+        if (e == b) {
+            empty_row[r - nzpos[r]] = (int32_t)r;
+            continue;
+        }
+        nz_row[nzpos[r]] = (int32_t)r;
+        rv_col[e - 1] |= dev::kRowEnd;
         if (e - b <= thr)
             continue;
         const int64_t h = hubpos[r], s0 = segoff[r];
@@ -456,6 +471,7 @@ __global__ void hub_segments_kernel(const int64_t *ptr, int64_t N, int64_t thr, 
         for (int64_t q = b; q < e; q += seg, s++) {
             seg_row[s] = (int32_t)r;
             seg_beg[s] = q;
+            item[s] = dev::WorkItem{q, (int32_t)min(seg, e - q), 0};
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -596,17 +612,19 @@ __global__ void __launch_bounds__(kThreads) task_starts_kernel(const int64_t *pt
         start[base + j] = on[j] && ptr[base + j + 1] - ptr[base + j] <= thr;
 }
 
-// Task pos[r] of every row r with start[r]: rows [r, next(r)), without the hub
-// row that closed it.
+// Work item pos[r] of every row r with start[r]: the entries of rows
+// [r, next(r)), without the hub row that closed it.
 __global__ void task_write_kernel(const int64_t *ptr, const int32_t *next, int64_t N, int64_t thr,
-                                  const uint32_t *start, const uint32_t *pos, int32_t *rb, int32_t *re)
+                                  const uint32_t *start, const uint32_t *pos, const uint32_t *nzpos,
+                                  dev::WorkItem *item)
 {
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
         if (!start[r])
             continue;
-        const int64_t e = next[r];
-        rb[pos[r]] = (int32_t)r;
-        re[pos[r]] = (int32_t)(ptr[e] - ptr[e - 1] > thr ? e - 1 : e);
+        int64_t e = next[r];
+        if (ptr[e] - ptr[e - 1] > thr)
+            e--;
+        item[pos[r]] = dev::WorkItem{ptr[r], (int32_t)(ptr[e] - ptr[r]), (int32_t)nzpos[r]};
     }
 }
 
@@ -1028,7 +1046,7 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
         // columns, row pointers, hub and segment positions, the task packing's
         // row arrays, small values, the scans' block sums
         const size_t bytes = 2 * (8 * n + a) + 2 * (4 * n + a) + (4 * (size_t)ntiles * kBins + a) + 3 * (4 * n + a) +
-                             (8 * rows + a) + 7 * (4 * (rows + kTaskBlock) + a) + 6 * a + 24 * (4 * scan_blocks + a);
+                             (8 * rows + a) + 8 * (4 * (rows + kTaskBlock) + a) + 6 * a + 28 * (4 * scan_blocks + a);
         COLA_TRY(sc.reserve(bytes));
     }
     if (nnz > 0)
@@ -1073,12 +1091,13 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     }
     COLA_CUDA(cudaGetLastError());
     // hub rows and their segments; the tasks of the other rows
-    uint32_t nhub = 0, nseg = 0, ntask = 0;
-    uint32_t *hubpos = nullptr, *segoff = nullptr, *tstart = nullptr, *tpos = nullptr;
+    uint32_t nhub = 0, nseg = 0, ntask = 0, nnz_rows = 0;
+    uint32_t *hubpos = nullptr, *segoff = nullptr, *nzpos = nullptr, *tstart = nullptr, *tpos = nullptr;
     int32_t *tnext = nullptr, *texit = nullptr, *texit2 = nullptr, *tentry = nullptr, *tsuper = nullptr;
     const int64_t ntb = ((int64_t)N + kTaskBlock - 1) / kTaskBlock, nsuper = (ntb + kTaskSuper - 1) / kTaskSuper;
     COLA_TRY(sc.get(hubpos, N));
     COLA_TRY(sc.get(segoff, N));
+    COLA_TRY(sc.get(nzpos, N));
     COLA_TRY(sc.get(tnext, N));
     COLA_TRY(sc.get(texit, N));
     COLA_TRY(sc.get(tstart, N));
@@ -1088,6 +1107,7 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     COLA_TRY(sc.get(tsuper, nsuper));
     COLA_TRY(exclusive_scan(HubF{rv_ptr, thr}, N, hubpos, d_total, &nhub, sc));
     COLA_TRY(exclusive_scan(SegCountF{rv_ptr, thr, seg}, N, segoff, d_total, &nseg, sc));
+    COLA_TRY(exclusive_scan(SomeF{rv_ptr}, N, nzpos, d_total, &nnz_rows, sc));
     if (N > 0) {
         task_next_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(rv_ptr, N, thr, te, hubpos, tnext);
         task_exit_kernel<<<(unsigned)ntb, kThreads, 0, st>>>(tnext, N, texit);
@@ -1121,7 +1141,11 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     const size_t o_ptr = place(((size_t)N + 1) * 8), o_col = place((size_t)U * 4), o_val = place((size_t)U * 4);
     const size_t o_srow = place((size_t)nseg * 4), o_sbeg = place((size_t)nseg * 8);
     const size_t o_hrow = place((size_t)nhub * 4), o_hseg = place(((size_t)nhub + 1) * 8);
-    const size_t o_trb = place((size_t)ntask * 4), o_tre = place((size_t)ntask * 4);
+    const int64_t nempty = (int64_t)N - nnz_rows, nitem = (int64_t)nseg + ntask;
+    COLA_REQUIRE(nitem < INT32_MAX, COLA_ERROR_UNSUPPORTED, "%s: %lld work items (2^31 at most)", who,
+                 (long long)nitem);
+    const size_t o_item = place((size_t)nitem * sizeof(dev::WorkItem));
+    const size_t o_nz = place(((size_t)nnz_rows + dev::kRowPad) * 4), o_empty = place((size_t)nempty * 4);
     const size_t qbytes = (dev::kMaxItemQueues + 1) * sizeof(unsigned int), o_q = place(qbytes);
     total = std::max<size_t>(total, 256);
     COLA_CUDA(cudaMalloc(&g->dmem, total));
@@ -1135,15 +1159,17 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     }
     const int64_t *ptr_final = reinterpret_cast<const int64_t *>(base + o_ptr);
     if (N > 0) {
-        hub_segments_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(
-            ptr_final, N, thr, seg, hubpos, segoff, nhub, nseg, reinterpret_cast<int32_t *>(base + o_hrow),
+        dev::WorkItem *item = reinterpret_cast<dev::WorkItem *>(base + o_item);
+        int32_t *nz_row = reinterpret_cast<int32_t *>(base + o_nz);
+        COLA_CUDA(cudaMemsetAsync(nz_row + nnz_rows, 0, dev::kRowPad * 4, st));
+        rows_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(
+            ptr_final, N, thr, seg, hubpos, segoff, nzpos, nhub, nseg, reinterpret_cast<int32_t *>(base + o_hrow),
             reinterpret_cast<int64_t *>(base + o_hseg), reinterpret_cast<int32_t *>(base + o_srow),
-            reinterpret_cast<int64_t *>(base + o_sbeg));
-        t_launches++;
-        task_write_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(ptr_final, tnext, N, thr, tstart, tpos,
-                                                                 reinterpret_cast<int32_t *>(base + o_trb),
-                                                                 reinterpret_cast<int32_t *>(base + o_tre));
-        t_launches++;
+            reinterpret_cast<int64_t *>(base + o_sbeg), item, nz_row, reinterpret_cast<int32_t *>(base + o_empty),
+            reinterpret_cast<int32_t *>(base + o_col));
+        task_write_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(ptr_final, tnext, N, thr, tstart, tpos, nzpos,
+                                                                 item + nseg);
+        t_launches += 2;
         COLA_CUDA(cudaGetLastError());
     } else {
         const int64_t zero = 0;
@@ -1158,8 +1184,10 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     g->seg_beg = reinterpret_cast<const int64_t *>(base + o_sbeg);
     g->hub_row = reinterpret_cast<const int32_t *>(base + o_hrow);
     g->hub_seg = reinterpret_cast<const int64_t *>(base + o_hseg);
-    g->task_rb = reinterpret_cast<const int32_t *>(base + o_trb);
-    g->task_re = reinterpret_cast<const int32_t *>(base + o_tre);
+    g->items = base + o_item;
+    g->nz_row = reinterpret_cast<const int32_t *>(base + o_nz);
+    g->empty_row = reinterpret_cast<const int32_t *>(base + o_empty);
+    g->nempty = nempty;
     g->item_queue = reinterpret_cast<unsigned int *>(base + o_q);
     g->nseg = nseg;
     g->nhub = nhub;

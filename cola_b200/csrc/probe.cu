@@ -80,12 +80,12 @@ __global__ void __launch_bounds__(256) graph_gather_kernel(const char *__restric
     const int64_t nwarps = (int64_t)gridDim.x * 8;
     uint32_t acc = 0;
     // the next batch of indices is loaded while this one's rows are read
-    int32_t next = warp * 32 + lane < nnz ? __ldcs(col + warp * 32 + lane) : 0;
+    int32_t next = warp * 32 + lane < nnz ? __ldcs(col + warp * 32 + lane) & dev::kColMask : 0;
     for (int64_t e0 = warp * 32; e0 < nnz; e0 += nwarps * 32) {
         const int n = (int)min((int64_t)32, nnz - e0);
         const int32_t mine = next;
         const int64_t e1 = e0 + nwarps * 32 + lane;
-        next = e1 < nnz ? __ldcs(col + e1) : 0;
+        next = e1 < nnz ? __ldcs(col + e1) & dev::kColMask : 0;
         for (int j = 0; j < n; j += 4) {
             uint4 v[4][VECS];
 #pragma unroll

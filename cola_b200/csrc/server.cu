@@ -183,7 +183,6 @@ static cola_status launch_group(cola_server *S, Group *G)
     COLA_REQUIRE(n <= sl.cap, COLA_ERROR_INVALID_ARGUMENT, "server: group of %d exceeds the slot's %d", n, sl.cap);
     const Request *r0 = G->reqs[0];
     const size_t xs = r0->xdt == COLA_FLOAT32 ? 4 : 2, ys = r0->ydt == COLA_FLOAT32 ? 4 : 2;
-    int64_t items = 0, hub = 0;
     // a small group moves its bytes with the SMs when every host buffer allows it
     bool by_sms = G->small && S->sm_copies && sm_copy_ok(sl.h_desc, sl.d_desc, 16);
     for (const Request *r : G->reqs)
@@ -205,21 +204,15 @@ static cola_status launch_group(cola_server *S, Group *G)
                                   S->copy_chunk, st));
         BatchGraph &d = sl.h_desc[i];
         fill_batch_graph(d, g, r->dX, r->K, r->dY, r->K, r->K, r->xdt, r->dws);
-        d.item0 = items;
-        d.hub0 = hub;
-        items += g->nseg + g->ntask;
-        hub += g->nhub * ((r->K + 127) / 128);
     }
+    BatchLaunch L = {};
+    COLA_TRY(build_groups(sl.h_desc, (int)n, L));
     COLA_CUDA(cudaEventRecord(sl.ev[1], st));
     if (by_sms && ((size_t)n * sizeof(BatchGraph)) % 16 == 0)
         COLA_TRY(copy_by_sms(sl.d_desc, sl.h_desc, (size_t)n * sizeof(BatchGraph), false, st));
     else
         COLA_CUDA(cudaMemcpyAsync(sl.d_desc, sl.h_desc, (size_t)n * sizeof(BatchGraph), cudaMemcpyHostToDevice, st));
-    BatchLaunch L;
     L.desc = sl.d_desc;
-    L.ngraphs = n;
-    L.total_items = items;
-    L.total_hub = hub;
     L.xdt = r0->xdt;
     L.ydt = r0->ydt;
     L.unroll = 4;

@@ -20,6 +20,7 @@
 #include "graph.h"
 #include "spmm_kernels.cuh"
 #include "spmm_rows.cuh"
+#include "batch.h"
 
 using cola::dev::GatherSeg;
 using cola::dev::PartDesc;
@@ -362,7 +363,7 @@ static cola_status launch_rows(const RowsLaunch &a, cudaStream_t st)
                  : launch_rows_geo<dev::ScalarTraits<BF>, BF, false>(a, a.K, st);
 }
 
-template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC, int MINB = 1>
+template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB = 1>
 static cola_status launch_block_t(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
 {
     using T = typename dev::ElemOf<TR>::T;
@@ -372,32 +373,20 @@ static cola_status launch_block_t(const dev::BlockArgs &ba, const RowsLaunch &a,
         if (a.k_tile > 0 && ntile > 1) {
             // a requested tile width: one grid sweeps the tiles one after another
             auto fn = dev::rowblock_tiled_kernel<TR, TY, NV, UNROLL, MINB>;
-            const int64_t gx = grid_for((const void *)fn, (ba.nseg + ba.ntask) * ntile);
             t_launches++;
-            fn<<<(unsigned)gx, dev::kThreads, 0, st>>>(ba, static_cast<const T *>(a.X), a.ldx,
-                                                       static_cast<TY *>(a.Y), a.ldy, a.K, a.accumulate);
-            COLA_CUDA(cudaGetLastError());
+            COLA_CUDA(launch_kernel(fn, (unsigned)grid_for((const void *)fn, ba.nitem * ntile), 1, false, st, ba,
+                                    static_cast<const T *>(a.X), a.ldx, static_cast<TY *>(a.Y), a.ldy, a.K,
+                                    a.accumulate));
             return COLA_SUCCESS;
         }
     }
-    if (ba.queue && ntile <= dev::kMaxItemQueues) {
-        // items drawn from the graph's counters: a warp that met slow items draws fewer
-        auto fn = dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, VEC, MINB, true>;
-        const int64_t gx = grid_for((const void *)fn, ba.nseg + ba.ntask);
-        t_launches++;
-        fn<<<dim3((unsigned)gx, (unsigned)ntile), dev::kThreads, 0, st>>>(ba, static_cast<const T *>(a.X), a.ldx,
-                                                                          static_cast<TY *>(a.Y), a.ldy, a.K,
-                                                                          a.accumulate);
-        COLA_CUDA(cudaGetLastError());
-        return COLA_SUCCESS;
-    }
-    auto fn = dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, VEC, MINB>;
-    const int64_t gx = grid_for((const void *)fn, ba.nseg + ba.ntask);
+    // items drawn from the graph's counters: a warp that met slow items draws fewer
+    const bool dyn = ba.queue && ntile <= dev::kMaxItemQueues;
+    auto fn = dyn ? dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, true>
+                  : dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, false>;
     t_launches++;
-    fn<<<dim3((unsigned)gx, (unsigned)ntile), dev::kThreads, 0, st>>>(ba, static_cast<const T *>(a.X), a.ldx,
-                                                                      static_cast<TY *>(a.Y), a.ldy, a.K,
-                                                                      a.accumulate);
-    COLA_CUDA(cudaGetLastError());
+    COLA_CUDA(launch_kernel(fn, (unsigned)grid_for((const void *)fn, ba.nitem), (unsigned)ntile, false, st, ba,
+                            static_cast<const T *>(a.X), a.ldx, static_cast<TY *>(a.Y), a.ldy, a.K, a.accumulate));
     return COLA_SUCCESS;
 }
 
@@ -409,16 +398,16 @@ static cola_status launch_block_narrow(const dev::BlockArgs &ba, const RowsLaunc
     const int mb = a.min_blocks == 6 || a.min_blocks == 8 ? a.min_blocks : 4;
     if (a.unroll == 8) {
         if (mb == 8)
-            return launch_block_t<TR, TY, 32, 1, 8, true, 8>(ba, a, st);
+            return launch_block_t<TR, TY, 32, 1, 8, 8>(ba, a, st);
         if (mb == 6)
-            return launch_block_t<TR, TY, 32, 1, 8, true, 6>(ba, a, st);
-        return launch_block_t<TR, TY, 32, 1, 8, true, 4>(ba, a, st);
+            return launch_block_t<TR, TY, 32, 1, 8, 6>(ba, a, st);
+        return launch_block_t<TR, TY, 32, 1, 8, 4>(ba, a, st);
     }
     if (mb == 8)
-        return launch_block_t<TR, TY, 32, 1, 4, true, 8>(ba, a, st);
+        return launch_block_t<TR, TY, 32, 1, 4, 8>(ba, a, st);
     if (mb == 6)
-        return launch_block_t<TR, TY, 32, 1, 4, true, 6>(ba, a, st);
-    return launch_block_t<TR, TY, 32, 1, 4, true, 4>(ba, a, st);
+        return launch_block_t<TR, TY, 32, 1, 4, 6>(ba, a, st);
+    return launch_block_t<TR, TY, 32, 1, 4, 4>(ba, a, st);
 }
 
 // V = 16-byte vectors per row: LG lanes per row tile, G = 32/LG lane groups.
@@ -426,39 +415,36 @@ template <typename TR, typename TY>
 static cola_status launch_block_geo(const dev::BlockArgs &ba, const RowsLaunch &a, int V, cudaStream_t st)
 {
     if (V <= 1)
-        return launch_block_t<TR, TY, 1, 1, 1, true>(ba, a, st);
+        return launch_block_t<TR, TY, 1, 1, 1, 4>(ba, a, st);
     if (V <= 2)
-        return launch_block_t<TR, TY, 2, 1, 2, true>(ba, a, st);
+        return launch_block_t<TR, TY, 2, 1, 2, 4>(ba, a, st);
     if (V <= 4)
-        return launch_block_t<TR, TY, 4, 1, 4, true, 4>(ba, a, st);
+        return launch_block_t<TR, TY, 4, 1, 4, 4>(ba, a, st);
     if (V <= 8)
-        return launch_block_t<TR, TY, 8, 1, 4, true, 4>(ba, a, st);
+        return launch_block_t<TR, TY, 8, 1, 4, 4>(ba, a, st);
     if (V <= 16)
-        return launch_block_t<TR, TY, 16, 1, 4, true, 4>(ba, a, st);
+        return launch_block_t<TR, TY, 16, 1, 4, 4>(ba, a, st);
     if (V <= 32) {
-        if (a.unroll == 8)
-            return launch_block_t<TR, TY, 32, 1, 8, true>(ba, a, st);
+        if (a.unroll == 6 || a.unroll == 8)  // rounds divide the 32-entry batch
+            return launch_block_t<TR, TY, 32, 1, 8>(ba, a, st);
         if (a.unroll == 2)
-            return launch_block_t<TR, TY, 32, 1, 2, true>(ba, a, st);
-        if (a.unroll == 6)
-            return launch_block_t<TR, TY, 32, 1, 6, true>(ba, a, st);
-        // resident blocks per SM: measured best 3 for FP32 X (K = 128: 3 % faster
-        // than 4) and 4 for BF16 X (5 % faster than 3)
-        const int mb = a.min_blocks > 0 ? a.min_blocks : (TR::E == 4 ? 3 : 4);
+            return launch_block_t<TR, TY, 32, 1, 2>(ba, a, st);
+        const int mb = a.min_blocks > 0 ? a.min_blocks : 4;
         if (mb == 3)
-            return launch_block_t<TR, TY, 32, 1, 4, true, 3>(ba, a, st);
+            return launch_block_t<TR, TY, 32, 1, 4, 3>(ba, a, st);
         if (mb == 5)
-            return launch_block_t<TR, TY, 32, 1, 4, true, 5>(ba, a, st);
+            return launch_block_t<TR, TY, 32, 1, 4, 5>(ba, a, st);
         if (mb == 6)
-            return launch_block_t<TR, TY, 32, 1, 4, true, 6>(ba, a, st);
-        return launch_block_t<TR, TY, 32, 1, 4, true, 4>(ba, a, st);
+            return launch_block_t<TR, TY, 32, 1, 4, 6>(ba, a, st);
+        return launch_block_t<TR, TY, 32, 1, 4, 4>(ba, a, st);
     }
-    if (V <= 64) {
-        if (a.unroll == 4 || a.unroll == 8)
-            return launch_block_t<TR, TY, 32, 2, 4, true>(ba, a, st);
-        return launch_block_t<TR, TY, 32, 2, 2, true>(ba, a, st);
-    }
-    return launch_block_t<TR, TY, 32, 4, 2, true>(ba, a, st);
+    // rows wider than one vector a lane: two vectors, tiles of 64 vectors side by
+    // side.  R-MAT, 262 K rows, 5.5 M entries, K = 512 FP32: 0.69 ms with 4 rows in
+    // flight at 3 blocks, 0.75 with 2 at 4 blocks, 0.72 with one vector a lane,
+    // 0.79 with four (2 rows in flight, 2 blocks).
+    if (a.unroll == 2)
+        return launch_block_t<TR, TY, 32, 2, 2, 4>(ba, a, st);
+    return launch_block_t<TR, TY, 32, 2, 4, 3>(ba, a, st);
 }
 
 // Feature tile of one pass for the requested k_tile (0 = the library's
@@ -477,10 +463,8 @@ static int rows_k_tile(cola_dtype xdt, int K, int k_tile)
 // Row-block streaming launch (vector path).
 static cola_status launch_block(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
 {
-    if (ba.nseg + ba.ntask <= 0)
+    if (ba.nitem <= 0)
         return COLA_SUCCESS;
-    COLA_REQUIRE(ba.nseg + ba.ntask < INT32_MAX, COLA_ERROR_UNSUPPORTED, "cola_spmm: %lld work items (2^31 at most)",
-                 (long long)(ba.nseg + ba.ntask));
     using BF = __nv_bfloat16;
     const int kt = rows_k_tile(a.xdt, a.K, a.k_tile);
     if (kt > 0) {
@@ -516,7 +500,7 @@ bool vec_ok_rows(cola_dtype xdt, const void *X, int64_t ldx, cola_dtype ydt, con
 {
     const int E = xdt == COLA_FLOAT32 ? 4 : 8;
     const int ysz = ydt == COLA_FLOAT32 ? 4 : 2;
-    if (K % E || ldx % E || ldx > INT32_MAX || !aligned16(X))
+    if (K % E || ldx % E || ldx > INT32_MAX / (xdt == COLA_FLOAT32 ? 4 : 2) || !aligned16(X))
         return false;
     if (ldy % E || ((uintptr_t)Y % (uintptr_t)(E * ysz)) != 0)
         return false;
@@ -840,6 +824,7 @@ cola_status graph_upload(const cola_partition_set *ps, const cola_upload_opts *o
     // entries in ascending global column order, hub segments, row tasks
     const bool rows = !(opts && opts->no_row_view);
     RowView rv;
+    RowItems ri;
     if (rows) {
         int64_t nnz_all = 0;
         for (const PartHost &ph : ps->parts)
@@ -852,6 +837,11 @@ cola_status graph_upload(const cola_partition_set *ps, const cola_upload_opts *o
         g->nseg = (int64_t)rv.seg_row.size();
         g->nhub = (int64_t)rv.hub_row.size();
         g->ntask = (int64_t)rv.task_rb.size();
+        static_assert(sizeof(RowItem) == sizeof(dev::WorkItem), "the same 16 bytes on host and device");
+        build_row_items(rv, g->hub_segment, dev::kRowEnd, dev::kRowPad, ri);
+        g->nempty = (int64_t)ri.empty_row.size();
+        COLA_REQUIRE(ri.item.size() < (size_t)INT32_MAX, COLA_ERROR_UNSUPPORTED,
+                     "cola_graph_upload: %zu work items (2^31 at most)", ri.item.size());
     }
 
     // one device allocation for everything
@@ -900,7 +890,7 @@ cola_status graph_upload(const cola_partition_set *ps, const cola_upload_opts *o
     }
     const size_t desc_buf = ar.add(nullptr, (size_t)P * sizeof(GatherSeg));
     size_t o_rv_ptr = 0, o_rv_col = 0, o_rv_val = 0, o_seg_row = 0, o_seg_beg = 0, o_hub_row = 0, o_hub_seg = 0;
-    size_t o_task_rb = 0, o_task_re = 0, o_queue = 0;
+    size_t o_item = 0, o_nz = 0, o_empty = 0, o_queue = 0;
     if (rows) {
         o_rv_ptr = ar.add(rv.ptr.data(), rv.ptr.size() * 8);
         o_rv_col = ar.add(rv.col.data(), rv.col.size() * 4);
@@ -909,8 +899,9 @@ cola_status graph_upload(const cola_partition_set *ps, const cola_upload_opts *o
         o_seg_beg = ar.add(rv.seg_beg.data(), rv.seg_beg.size() * 8);
         o_hub_row = ar.add(rv.hub_row.data(), rv.hub_row.size() * 4);
         o_hub_seg = ar.add(rv.hub_seg.data(), rv.hub_seg.size() * 8);
-        o_task_rb = ar.add(rv.task_rb.data(), rv.task_rb.size() * 4);
-        o_task_re = ar.add(rv.task_re.data(), rv.task_re.size() * 4);
+        o_item = ar.add(ri.item.data(), ri.item.size() * sizeof(RowItem));
+        o_nz = ar.add(ri.nz_row.data(), ri.nz_row.size() * 4);
+        o_empty = ar.add(ri.empty_row.data(), ri.empty_row.size() * 4);
         o_queue = ar.add(nullptr, (dev::kMaxItemQueues + 1) * sizeof(unsigned int));  // zero in the image
     }
     ar.total = std::max<size_t>(ar.total, 256);
@@ -927,8 +918,9 @@ cola_status graph_upload(const cola_partition_set *ps, const cola_upload_opts *o
         g->seg_beg = reinterpret_cast<const int64_t *>(base + o_seg_beg);
         g->hub_row = at(o_hub_row);
         g->hub_seg = reinterpret_cast<const int64_t *>(base + o_hub_seg);
-        g->task_rb = at(o_task_rb);
-        g->task_re = at(o_task_re);
+        g->items = base + o_item;
+        g->nz_row = at(o_nz);
+        g->empty_row = at(o_empty);
         g->item_queue = reinterpret_cast<unsigned int *>(base + o_queue);
     }
 
@@ -1215,38 +1207,22 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         a.min_blocks = opts ? opts->min_blocks : 0;
         a.k_tile = opts ? opts->k_tile : 0;
         if (a.vec) {
-            dev::BlockArgs ba;
-            ba.rowptr = g->rv_ptr;
-            ba.col = g->rv_col;
-            ba.val = g->rv_val;
-            ba.task_rb = g->task_rb;
-            ba.task_re = g->task_re;
-            ba.ntask = g->ntask;
-            ba.seg_row = g->seg_row;
-            ba.seg_beg = g->seg_beg;
-            ba.nseg = g->nseg;
-            ba.seg_len = g->hub_segment;
-            ba.ws = g->ws_hub;
-            ba.ld_ws = K;
-            ba.queue = g->item_queue;
-            COLA_TRY(launch_block(ba, a, st));
+            COLA_TRY(launch_block(block_args(g, g->ws_hub, K), a, st));
         } else {
             COLA_TRY(launch_rows(a, st));
         }
         if (g->nhub > 0 && a.vec && K % 4 == 0 && ldy % 4 == 0 &&
             aligned16(g->ws_hub) && ((uintptr_t)Y % (ydt == COLA_FLOAT32 ? 16 : 8)) == 0) {
-            const int64_t items = g->nhub * ((K + 127) / 128);
-            const int64_t blocks = std::min<int64_t>((items + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock,
-                                                     (int64_t)sm_count() * 16);
+            const unsigned blocks = hub_blocks(g->nhub * dev::hub_tiles(K), dev::hub_lanes(K));
             t_launches++;
             if (ydt == COLA_FLOAT32)
-                dev::hub_combine_vec_kernel<float, 4><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, K, static_cast<float *>(Y), ldy, K, accumulate);
+                COLA_CUDA(launch_kernel(dev::hub_combine_vec_kernel<float>, blocks, 1, true, st, g->hub_row,
+                                        g->hub_seg, g->nhub, g->ws_hub, K, static_cast<float *>(Y), ldy, K,
+                                        accumulate));
             else
-                dev::hub_combine_vec_kernel<__nv_bfloat16, 4><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, K, static_cast<__nv_bfloat16 *>(Y), ldy, K,
-                    accumulate);
-            COLA_CUDA(cudaGetLastError());
+                COLA_CUDA(launch_kernel(dev::hub_combine_vec_kernel<__nv_bfloat16>, blocks, 1, true, st, g->hub_row,
+                                        g->hub_seg, g->nhub, g->ws_hub, K, static_cast<__nv_bfloat16 *>(Y), ldy, K,
+                                        accumulate));
         } else if (g->nhub > 0) {
             const int64_t blocks = (g->nhub + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock;
             t_launches++;

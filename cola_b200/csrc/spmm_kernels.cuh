@@ -24,6 +24,12 @@ constexpr int kThreads = kWarpsPerBlock * 32;
 // Row-major schedule: feature tiles (gridDim.y) that can draw work items from
 // counters of their own; a graph holds kMaxItemQueues + 1 counters.
 constexpr int kMaxItemQueues = 64;
+// Row view on the device: the sign bit of an entry's column marks the last
+// entry of its row (column ids are below 2^31).
+constexpr int32_t kRowEnd = INT32_MIN;
+constexpr int32_t kColMask = INT32_MAX;
+// Padding of the list of rows with entries (read 32 at a time).
+constexpr int kRowPad = 32;
 
 // Where a remote chunk's dense row comes from.
 enum RemoteMode : int32_t {

@@ -1,16 +1,18 @@
 // Row-major ("one writer per output row") schedule of the partitioned SpMM.
 //
 // At upload every partition's remote CSC block is transposed and merged with
-// its local CSR, giving for each output row its entries in column order.  One
-// warp owns one row: it gathers the rows of X its entries name (16-byte
-// vectors, UNROLL loads in flight per lane group), accumulates in FP32
-// registers and writes the output row once with plain stores — no atomics, no
+// its local CSR, giving for each output row its entries in column order.
+// Warps stream work items -- runs of rows, or segments of rows longer than a
+// threshold ("hubs") -- gather the rows of X the entries name (16-byte
+// vectors, UNROLL loads in flight per lane group), accumulate in FP32
+// registers and write each output row once with plain stores: no atomics, no
 // zeroing pass, the same summation order on every run, and BF16 output is
-// rounded straight from the registers.  Rows longer than a threshold ("hubs")
-// are cut into fixed-length segments processed by separate warps into an FP32
-// workspace; a second kernel adds each hub's segment partials pairwise (a
-// binary tree in fixed order) and writes the row.
+// rounded straight from the registers.  Hub segments go to an FP32 workspace;
+// a second kernel adds each hub's partials pairwise (a binary tree in fixed
+// order) and writes the row.
 #pragma once
+#include <type_traits>
+
 #include "spmm_kernels.cuh"
 
 namespace cola {
@@ -97,7 +99,7 @@ __device__ __forceinline__ void store_out<__nv_bfloat16, 1, false>(__nv_bfloat16
 // rowptr[row[s]+1])) and writes its partial to ws row s.
 struct RowsArgs {
     const int64_t *rowptr;  // N+1
-    const int32_t *col;     // global column ids
+    const int32_t *col;     // global column ids (kRowEnd on a row's last entry)
     const float *val;
     int32_t nrows;
     int32_t hub_threshold;  // rows with more entries are handled by segments
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(kThreads) rows_spmm_kernel(const __grid_consta
             int mc = 0;
             float mv = 0.f;
             if (lane < n) {
-                mc = __ldg(ra.col + base + lane);
+                mc = __ldg(ra.col + base + lane) & kColMask;
                 mv = __ldg(ra.val + base + lane);
             }
             for (int jj = 0; jj < n; jj += G * UNROLL) {
@@ -221,25 +223,30 @@ __global__ void __launch_bounds__(kThreads) rows_spmm_kernel(const __grid_consta
     }
 }
 
-// Row-block streaming form of the same schedule, for rows one warp wide
-// (LG = 32).  A task is a contiguous block of rows holding about the same
-// number of entries as every other task (hub rows excluded: they come as
-// segments).  The warp streams the block's entries as one flat list -- index
-// batch b+1 is loaded while batch b is consumed, UNROLL rows of X are in flight
-// -- and flushes the running sums to the output row whenever the stream
-// crosses a row end, writing empty rows as zeros.  Loads therefore keep flowing
-// across row boundaries instead of restarting a dependent chain per row.
+// Work items of the streaming form, segments first, then tasks, one 16-byte
+// descriptor each (a dependent chain of row pointers per item otherwise):
+//   segment it:  entries [beg, beg + n) of one hub row; partial -> ws row it
+//   task:        entries [beg, beg + n) of consecutive rows; out = position in
+//                nz_row of the first of its rows that has entries
+// An entry's column carries kRowEnd when it is the last of its row, so the
+// stream needs no row pointers.  Rows without entries are in no item: every
+// item writes its even share of their zeros at its end, beside other warps'
+// gathers (0.04 of 1.07 ms on a scale-20 R-MAT graph at K = 128).
+struct __align__(16) WorkItem {
+    int64_t beg;
+    int32_t n;
+    int32_t out;
+};
+
 struct BlockArgs {
-    const int64_t *rowptr;
+    const WorkItem *item;
     const int32_t *col;
     const float *val;
-    const int32_t *task_rb, *task_re;  // task t: rows [task_rb[t], task_re[t])
-    int64_t ntask;
-    const int32_t *seg_row;
-    const int64_t *seg_beg;
-    int64_t nseg;
-    int32_t seg_len;
-    float *ws;
+    const int32_t *nz_row;     // rows with entries, ascending
+    const int32_t *empty_row;  // rows without, ascending
+    int32_t nseg, nitem;  // items [0, nseg) segments, [nseg, nitem) tasks
+    int32_t nempty, empty_share;  // rows without entries, and how many of them an item writes
+    float *ws;            // nseg x K FP32 partials
     int64_t ld_ws;
     // Work-item counters for the dynamic schedule (kMaxItemQueues per-tile
     // counters, then the count of warps that have finished); all zero between
@@ -248,309 +255,433 @@ struct BlockArgs {
     unsigned int *queue;
 };
 
-// acc[q] += v * x[2q .. 2q+1] for one 16-byte vector of X, with the packed
-// FP32x2 fused multiply-add of sm_100 (two products per instruction).
+// acc[q] += v * x[2q .. 2q+1] for one vector of X, with the packed FP32x2
+// fused multiply-add of sm_100 (two products per instruction).
 template <typename TR>
-__device__ __forceinline__ void fma_vec2(float2 (&acc)[TR::E / 2], float v, const typename TR::raw_t &r)
+__device__ __forceinline__ void fma_vec2(float2 (&acc)[TR::E / 2], float2 vv, const typename TR::raw_t &r)
 {
     float f[TR::E];
     TR::unpack(r, f);
-    const float2 vv = make_float2(v, v);
 #pragma unroll
     for (int q = 0; q < TR::E / 2; q++)
         acc[q] = __ffma2_rn(vv, make_float2(f[2 * q], f[2 * q + 1]), acc[q]);
 }
 
-// LG lanes cover one row tile of X (NV vectors each); G = 32 / LG lane groups
-// of the warp take interleaved entries of the same stream (group g takes
-// entries g, g + G, ...), so narrow rows still keep 32 lanes busy.  A round is
-// G * UNROLL consecutive entries: when it lies inside the current output row
-// every group just accumulates; otherwise it is cut at the row ends, and at
-// every row end the groups' partial sums are added with __shfl_xor_sync and
-// group 0 writes the row.
-// Work items it0, it0 + stride, ... (< total) of the streaming schedule, each a
-// row-block task (rows [task_rb, task_re) of ba) or a hub segment (its partial
-// goes to ws row `it`); items count segments first, then tasks.  k0 is the
-// first feature of this call's tile; ent is the warp's 32-entry shared-memory
-// index batch.
-// LG > 0 fixes the lane-group width at compile time; LG == 0 takes it from
-// lg_rt at run time (8, 16 or 32), as the batched form does per graph.
-// BARef is `const BlockArgs` (the single-graph kernel: arguments read straight
-// from the kernel's parameter space) or `const BlockArgs &` (the batched form:
-// a descriptor in global memory).
-template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC_Y, typename BARef = const BlockArgs,
-          bool DYN = false>
-__device__ __forceinline__ void rowblock_items(BARef ba, const int64_t it0, const int64_t stride,
-                                               const int64_t total,
-                                              const typename ElemOf<TR>::T *__restrict__ X, const int64_t ldx,
-                                              TY *__restrict__ Y, const int64_t ldy, const int K, const int accumulate,
-                                              const int k0, int2 *ent, const int lg_rt = 0,
-                                              unsigned int *queue = nullptr)
+__device__ __forceinline__ WorkItem load_item(const WorkItem *p)
 {
+    const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
+    WorkItem w;
+    w.beg = (int64_t)(((uint64_t)(uint32_t)v.y << 32) | (uint32_t)v.x);
+    w.n = v.z;
+    w.out = v.w;
+    return w;
+}
+
+// The current 32 entries of a warp: columns and values apart, so that 4 columns
+// of a round are one 16-byte shared-memory load; each value twice, so that it
+// is read as the register pair the packed FMA takes; and the output rows that
+// end in the batch, in order.
+struct __align__(16) EntryBatch {
+    float2 val[32];
+    int32_t col[32];
+    int32_t row[32];
+};
+
+// base + c * stride bytes, one multiply-add.
+__device__ __forceinline__ const char *row_at(const char *base, int32_t c, int32_t stride)
+{
+    unsigned long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(c), "r"(stride), "l"(base));
+    return reinterpret_cast<const char *>(r);
+}
+
+// Lane id as a value the compiler keeps (it re-reads threadIdx, a slow special
+// register, inside the loops otherwise).
+__device__ __forceinline__ int lane_id()
+{
+    int l;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
+    return l;
+}
+
+// How an item's entries are summed: LG lanes cover one row tile of X (NV
+// vectors each); G = 32 / LG lane groups take interleaved entries of the stream
+// (group g takes entries g, g + G, ... of each 32-entry batch), so narrow rows
+// still keep 32 lanes busy.  A round is G * UNROLL consecutive entries whose
+// loads are all in flight; it is added up and cut where rows end.  At a row end
+// the groups' sums are added in a butterfly that halves the features each lane
+// holds at every step (about E shuffles a row instead of E log2 G), and each
+// lane writes the features it is left with.
+// What bounds it: the L1/L2 gather traffic of X with UNROLL x resident warps
+// rows in flight; instruction issue comes next, so a round inside one row costs
+// 3 shared loads, one address and one load per entry, and the products.
+// Measured (R-MAT, one lane group a row): scale 20, K = 128 FP32 1.11 -> 1.07 ms
+// against the form that walked row pointers, scale 21, K = 256 BF16 4.03 ->
+// 3.85, uniform rows of 20 entries at K = 100 83 -> 74 us; narrow rows: K = 16
+// BF16 206 -> 126 us, K = 32 FP32 on 16 K rows 23 -> 14 us.  Slower: 8 rows in
+// flight at 3 blocks (1.10 ms), 2 at 5 or 6 (1.35), the next row's load issued
+// as each row is added (1.64).
+template <typename TR, typename TY, int LG, int NV, int UNROLL>
+struct RowStream {
     using T = typename ElemOf<TR>::T;
     using raw_t = typename TR::raw_t;
-    constexpr int E = TR::E;
-    static_assert(LG == 0 || (32 / (LG > 0 ? LG : 1)) * UNROLL <= 32, "a round must fit in the 32-entry index batch");
-    const int lg = LG > 0 ? LG : lg_rt;
-    const int G = 32 / lg;
-    const int R = G * UNROLL;  // entries per round
-    const int lane = threadIdx.x & 31;
-    const int g = lane / lg;
-    const int gl = lane % lg;
+    static constexpr int E = TR::E;
+    static constexpr int G = 32 / LG;
+    static constexpr int R = G * UNROLL;  // entries per round
+    static constexpr int LANES = LG, NVEC = NV;
+    static_assert(32 % R == 0 && (NV == 1 || LG == 32), "rounds must divide the 32-entry batch");
+
+    float2 acc[NV][E / 2];
+    const char *xk;  // X + the lane's first feature
+    int32_t ldxb;    // bytes between rows (the vector path's fit 31 bits)
+    TY *Y;
+    int64_t ldy;
+    int koff;  // the lane's first feature
+    int lane, g, gl;
     bool kok[NV];
+    bool accumulate;
+
+    __device__ __forceinline__ void init(const T *X, int64_t ldx_, TY *Y_, int64_t ldy_, int K, int k0, int acc_)
+    {
+        lane = lane_id();
+        g = lane / LG;
+        gl = lane % LG;
+        ldxb = (int32_t)(ldx_ * (int64_t)sizeof(T));
+        ldy = ldy_;
+        koff = k0 + gl * E;
+        xk = reinterpret_cast<const char *>(X + koff);
+        Y = Y_;
+        accumulate = acc_ != 0;
 #pragma unroll
-    for (int j = 0; j < NV; j++)
-        kok[j] = (k0 + (gl + j * lg) * E) < K;
-    const T *xk = X + k0 + gl * E;
-    const int32_t ldx32 = (int32_t)ldx;  // the vector path's row stride fits 32 bits (one multiply-add per entry)
-
-    // DYN: items are drawn from a counter (lane 0, one item ahead, so the
-    // atomic's latency hides behind the current item); a warp that drew a
-    // slow item simply draws fewer.  Otherwise: it0, it0 + stride, ...
-    // Item numbers fit 32 bits (the launchers check nseg + ntask < 2^31): one
-    // register each, which keeps the 4-blocks-per-SM build within its 64.
-    const int32_t total32 = (int32_t)total;
-    int32_t it = (int32_t)it0;
-    if constexpr (DYN) {
-        unsigned int t = 0;
-        if (lane == 0)
-            t = atomicAdd(queue, 1u);
-        it = (int32_t)__shfl_sync(kFull, t, 0);
-    }
-    while (it < total32) {
-        unsigned int next_it = 0;
-        if constexpr (DYN) {
-            if (lane == 0)
-                next_it = atomicAdd(queue, 1u);
-        }
-        const bool seg = it < ba.nseg;
-        int32_t rb, re;
-        int64_t e_beg;
-        int32_t n_ent;  // entries of this item; indices below are relative to e_beg
-        if (seg) {
-            rb = __ldg(ba.seg_row + it);
-            re = rb + 1;
-            e_beg = __ldg(ba.seg_beg + it);
-            n_ent = (int32_t)min((int64_t)ba.seg_len, __ldg(ba.rowptr + rb + 1) - e_beg);
-        } else {
-            const int64_t t = it - ba.nseg;
-            rb = __ldg(ba.task_rb + t);
-            re = __ldg(ba.task_re + t);
-            e_beg = __ldg(ba.rowptr + rb);
-            n_ent = (int32_t)(__ldg(ba.rowptr + re) - e_beg);
-        }
-        const int32_t *colp = ba.col + e_beg;
-        const float *valp = ba.val + e_beg;
-        // ends of rows q0 .. q0+31, relative to e_beg (lane l: row q0 + l)
-        int32_t q0 = rb;
-        int32_t my_end = seg ? n_ent : (rb + lane < re ? (int32_t)(__ldg(ba.rowptr + rb + lane + 1) - e_beg) : n_ent);
-        int32_t cur = rb;
-        int32_t row_end = __shfl_sync(kFull, my_end, 0);
-
-        float2 acc[NV][E / 2];
-    #pragma unroll
         for (int j = 0; j < NV; j++)
-    #pragma unroll
+            kok[j] = koff + j * LG * E < K;
+    }
+
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int j = 0; j < NV; j++)
+#pragma unroll
             for (int q = 0; q < E / 2; q++)
                 acc[j][q] = make_float2(0.f, 0.f);
+    }
 
-        auto flush = [&]() {
-    #pragma unroll
-            for (int off = lg; off < 32; off <<= 1)
-    #pragma unroll
+    // The warp's sums to one row of Y or of the workspace (p: the lane's first
+    // feature in that row); clears them.
+    template <typename TO>
+    __device__ __forceinline__ void write_row(TO *p, bool add)
+    {
+        if constexpr (G == 1) {
+#pragma unroll
+            for (int j = 0; j < NV; j++) {
+                float a[E];
+#pragma unroll
+                for (int q = 0; q < E / 2; q++) {
+                    a[2 * q] = acc[j][q].x;
+                    a[2 * q + 1] = acc[j][q].y;
+                }
+                if (kok[j])
+                    store_out<TO, E, true>(p + j * LG * E, a, add);
+            }
+        } else {
+            float v[E];
+#pragma unroll
+            for (int q = 0; q < E / 2; q++) {
+                v[2 * q] = acc[0][q].x;
+                v[2 * q + 1] = acc[0][q].y;
+            }
+            // step `off`: the lane keeps the half its bit selects and adds the
+            // partner's, the same pairs in the same order as a full exchange
+            int f = 0;
+#pragma unroll
+            for (int off = LG, cnt = E; off < 32; off <<= 1, cnt = cnt > 1 ? cnt / 2 : 1) {
+                if (cnt > 1) {
+                    const bool up = (lane & off) != 0;
+#pragma unroll
+                    for (int q = 0; q < E / 2; q++)
+                        if (q < cnt / 2) {
+                            const float send = up ? v[q] : v[q + cnt / 2];
+                            const float keep = up ? v[q + cnt / 2] : v[q];
+                            v[q] = keep + __shfl_xor_sync(kFull, send, off);
+                        }
+                    f += up ? cnt / 2 : 0;
+                } else {
+                    v[0] += __shfl_xor_sync(kFull, v[0], off);
+                }
+            }
+            constexpr int EO = E / G > 0 ? E / G : 1;     // features a lane is left with
+            constexpr int kDup = E >= G ? 0 : 32 - LG * E;  // lane bits of the steps past one feature: copies
+            if (kok[0] && (lane & kDup) == 0) {
+                float a[EO];
+#pragma unroll
+                for (int q = 0; q < EO; q++)
+                    a[q] = v[q];
+                store_out<TO, EO, (EO > 1)>(p + f, a, add);
+            }
+        }
+        clear();
+    }
+
+    template <bool ALL>
+    __device__ __forceinline__ void load_round(const EntryBatch &eb, int jj, int cnt, raw_t (&xr)[UNROLL][NV]) const
+    {
+        int32_t c[UNROLL];
+        if constexpr (G == 1 && UNROLL % 4 == 0) {
+#pragma unroll
+            for (int u = 0; u < UNROLL; u += 4) {
+                const int4 v = *reinterpret_cast<const int4 *>(eb.col + jj + u);
+                c[u] = v.x;
+                c[u + 1] = v.y;
+                c[u + 2] = v.z;
+                c[u + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < UNROLL; u++)
+                c[u] = eb.col[jj + u * G + g];
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) {
+            if (ALL || u * G + g < cnt) {
+                const T *xp = reinterpret_cast<const T *>(row_at(xk, c[u], ldxb));
+#pragma unroll
                 for (int j = 0; j < NV; j++)
-    #pragma unroll
-                    for (int q = 0; q < E / 2; q++) {
-                        acc[j][q].x += __shfl_xor_sync(kFull, acc[j][q].x, off);
-                        acc[j][q].y += __shfl_xor_sync(kFull, acc[j][q].y, off);
-                    }
-            if (g == 0) {
-                if (seg) {
-                    // the segment's FP32 partial, read once by the combine kernel
-                    float *wp = ba.ws + (int64_t)it * ba.ld_ws + k0 + gl * E;
-    #pragma unroll
-                    for (int j = 0; j < NV; j++)
-                        if (kok[j]) {
-                            float a[E];
-    #pragma unroll
-                            for (int q = 0; q < E / 2; q++) {
-                                a[2 * q] = acc[j][q].x;
-                                a[2 * q + 1] = acc[j][q].y;
-                            }
-                            store_out<float, E, true>(wp + j * lg * E, a, false);
-                        }
-                } else {
-                    TY *yp = Y + (int64_t)cur * ldy + k0 + gl * E;
-    #pragma unroll
-                    for (int j = 0; j < NV; j++)
-                        if (kok[j]) {
-                            float a[E];
-    #pragma unroll
-                            for (int q = 0; q < E / 2; q++) {
-                                a[2 * q] = acc[j][q].x;
-                                a[2 * q + 1] = acc[j][q].y;
-                            }
-                            store_out<TY, E, VEC_Y>(yp + j * lg * E, a, accumulate != 0);
-                        }
-                }
+                    if (kok[j])
+                        xr[u][j] = TR::load(xp + j * LG * E);
             }
-    #pragma unroll
-            for (int j = 0; j < NV; j++)
-    #pragma unroll
-                for (int q = 0; q < E / 2; q++)
-                    acc[j][q] = make_float2(0.f, 0.f);
-            cur++;
-            if (!seg && cur < re) {
-                if (cur - q0 >= 32) {
-                    q0 += 32;
-                    my_end = q0 + lane < re ? (int32_t)(__ldg(ba.rowptr + q0 + lane + 1) - e_beg) : n_ent;
-                }
-                row_end = __shfl_sync(kFull, my_end, cur - q0);
-            }
-        };
+        }
+    }
 
-        int mc = 0;
-        float mv = 0.f;
-        if (lane < n_ent) {
-            // the entry stream is read once: evict-first, so it does not push X rows out of L2
-            mc = __ldcs(colp + lane);
-            mv = __ldcs(valp + lane);
-        }
-        for (int32_t base = 0; base < n_ent; base += 32) {
-            const int n = min(32, n_ent - base);
-            __syncwarp();
-            ent[lane] = make_int2(mc, __float_as_int(mv));
-            __syncwarp();
-            // prefetch the next index batch while this one is consumed
-            if (base + 32 + lane < n_ent) {
-                mc = __ldcs(colp + base + 32 + lane);
-                mv = __ldcs(valp + base + 32 + lane);
+    __device__ __forceinline__ void round_values(const EntryBatch &eb, int jj, float2 (&v)[UNROLL]) const
+    {
+        if constexpr (G == 1 && UNROLL % 2 == 0) {
+#pragma unroll
+            for (int u = 0; u < UNROLL; u += 2) {
+                const float4 w = *reinterpret_cast<const float4 *>(eb.val + jj + u);
+                v[u] = make_float2(w.x, w.y);
+                v[u + 1] = make_float2(w.z, w.w);
             }
-            for (int jj = 0; jj < n; jj += R) {
-                // the values are read from shared memory when the rows have
-                // arrived, not held in registers while the loads are in flight
-                raw_t xr[UNROLL][NV];
-                if (jj + R <= n && base + jj + R <= row_end) {
-                    // the whole round inside the current row: no boundary checks
-    #pragma unroll
-                    for (int u = 0; u < UNROLL; u++) {
-                        const T *xp = xk + (int64_t)ent[jj + u * G + g].x * ldx32;
-    #pragma unroll
+        } else {
+#pragma unroll
+            for (int u = 0; u < UNROLL; u++)
+                v[u] = eb.val[jj + u * G + g];
+        }
+    }
+
+    // One batch of n entries (1..32); ends: bit i set where entry i is its
+    // row's last.
+    __device__ __forceinline__ void batch(const EntryBatch &eb, const int n, const uint32_t ends)
+    {
+        int done = 0;
+        auto flush = [&]() {
+            const int row = eb.row[done++];
+            write_row(Y + (int64_t)row * ldy + koff, accumulate);
+        };
+#pragma unroll 1
+        for (int jj = 0; jj < n; jj += R) {
+            raw_t xr[UNROLL][NV];
+            const int cnt = min(R, n - jj);
+            uint32_t e = ends >> jj;
+            if (R < 32)
+                e &= (1u << (R & 31)) - 1u;
+            if (cnt == R)
+                load_round<true>(eb, jj, R, xr);
+            else
+                load_round<false>(eb, jj, cnt, xr);
+            float2 v[UNROLL];
+            round_values(eb, jj, v);
+            if (cnt == R && e == 0) {
+#pragma unroll
+                for (int u = 0; u < UNROLL; u++)
+#pragma unroll
+                    for (int j = 0; j < NV; j++)
+                        fma_vec2<TR>(acc[j], v[u], xr[u][j]);
+            } else if constexpr (G == 1 && UNROLL <= 4) {
+                // entry by entry: a row ends after the entries marked in e
+#pragma unroll
+                for (int u = 0; u < UNROLL; u++) {
+                    if (u < cnt) {
+#pragma unroll
                         for (int j = 0; j < NV; j++)
-                            if (kok[j])
-                                xr[u][j] = TR::load(xp + j * lg * E);
+                            fma_vec2<TR>(acc[j], v[u], xr[u][j]);
                     }
-    #pragma unroll
+                    if (e & (1u << u))
+                        flush();
+                }
+            } else {
+                // cut the round at the row ends it contains
+                int lo = 0;
+                while (true) {
+                    const int sh = e ? __ffs(e) : cnt;
+#pragma unroll
                     for (int u = 0; u < UNROLL; u++) {
-                        const float v = __int_as_float(ent[jj + u * G + g].y);
-    #pragma unroll
-                        for (int j = 0; j < NV; j++)
-                            fma_vec2<TR>(acc[j], v, xr[u][j]);
-                    }
-                } else {
-    #pragma unroll
-                    for (int u = 0; u < UNROLL; u++) {
-                        const int idx = jj + u * G + g;
-                        if (idx < n) {
-                            const T *xp = xk + (int64_t)ent[idx].x * ldx32;
-    #pragma unroll
+                        const int i = u * G + g;
+                        if (i >= lo && i < sh) {
+#pragma unroll
                             for (int j = 0; j < NV; j++)
-                                if (kok[j])
-                                    xr[u][j] = TR::load(xp + j * lg * E);
+                                fma_vec2<TR>(acc[j], v[u], xr[u][j]);
                         }
                     }
-                    // cut the round [lo, hi) at the row ends it contains
-                    int32_t lo = base + jj;
-                    const int32_t hi = base + jj + min(R, n - jj);
-                    while (true) {
-                        while (lo >= row_end)
-                            flush();
-                        const int32_t sh = min(row_end, hi);
-    #pragma unroll
-                        for (int u = 0; u < UNROLL; u++) {
-                            const int32_t e = base + jj + u * G + g;
-                            if (e >= lo && e < sh) {
-                                const float v = __int_as_float(ent[jj + u * G + g].y);
-    #pragma unroll
-                                for (int j = 0; j < NV; j++)
-                                    fma_vec2<TR>(acc[j], v, xr[u][j]);
-                            }
-                        }
-                        lo = sh;
-                        if (lo >= hi)
-                            break;
-                    }
+                    if (!e)
+                        break;
+                    flush();
+                    e &= e - 1;
+                    lo = sh;
+                    if (lo >= cnt)
+                        break;
                 }
             }
         }
-        while (cur < re)
-            flush();
-        if constexpr (DYN)
-            it = (int32_t)__shfl_sync(kFull, next_it, 0);
-        else
-            it += (int32_t)stride;
+    }
+};
+
+// One work item.  While a batch is summed the next one's entries are on their
+// way in registers.
+template <typename RS>
+__device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const int it, EntryBatch &eb)
+{
+    const int lane = rs.lane;
+    const bool seg = it < ba.nseg;
+    const WorkItem w = load_item(ba.item + it);
+    int64_t pos = w.beg + lane;
+    int left = w.n;
+    int kpos = w.out + lane;
+    int mc = 0, mr = 0;
+    float mv = 0.f;
+    auto fetch = [&]() {
+        // the entry stream is read once: evict-first, so it does not push X rows out of L2
+        if (lane < left) {
+            mc = __ldcs(ba.col + pos);
+            mv = __ldcs(ba.val + pos);
+        }
+        if (!seg)
+            mr = __ldg(ba.nz_row + kpos);  // the list is padded by 32
+    };
+    fetch();
+    rs.clear();
+    while (left > 0) {
+        const int n = min(32, left);
+        const uint32_t ends = seg ? 0u : __ballot_sync(kFull, mc < 0 && lane < n);
+        __syncwarp();
+        eb.col[lane] = mc & kColMask;
+        eb.val[lane] = make_float2(mv, mv);
+        eb.row[lane] = mr;
+        __syncwarp();
+        left -= 32;
+        pos += 32;
+        kpos += __popc(ends);
+        if (left > 0)
+            fetch();
+        rs.batch(eb, n, ends);
+    }
+    if (seg)
+        rs.write_row(ba.ws + (int64_t)it * ba.ld_ws + rs.koff, false);
+    // this item's share of the empty rows, G rows at a time
+    if (ba.nempty > 0 && !rs.accumulate) {
+        using TY = typename std::remove_pointer<decltype(rs.Y)>::type;
+        const int64_t z0 = (int64_t)it * ba.empty_share;
+        const int zn = (int)min((int64_t)ba.empty_share, ba.nempty - z0);
+        for (int i = rs.g; i < zn; i += RS::G) {
+            const int row = __ldg(ba.empty_row + z0 + i);
+            const float z[RS::E] = {};
+#pragma unroll
+            for (int j = 0; j < RS::NVEC; j++)
+                if (rs.kok[j])
+                    store_out<TY, RS::E, true>(rs.Y + (int64_t)row * rs.ldy + rs.koff + j * RS::LANES * RS::E, z, false);
+        }
+        __syncwarp();
     }
 }
 
-// End of a launch with the dynamic schedule: the last warp to finish puts the
-// item counters back to zero for the next launch (every warp has drawn its
-// final item before it counts itself finished).
-__device__ __forceinline__ void item_queue_release(unsigned int *queue)
+// The item after the one being drawn: the first one of every warp is its own
+// number, the others come from the counter.
+__device__ __forceinline__ unsigned int draw_item(unsigned int *queue, unsigned int nwarps)
+{
+    return nwarps + atomicAdd(queue, 1u);
+}
+
+// All items of one feature tile, drawn by this warp, one ahead, so that the
+// atomic's latency hides behind the current item.
+template <typename RS, bool DYN>
+__device__ __forceinline__ void stream_items(RS &rs, const BlockArgs &ba, const unsigned int warp,
+                                             const unsigned int nwarps, EntryBatch &eb,
+                                             unsigned int *queue)
+{
+    const unsigned int total = (unsigned int)ba.nitem;
+    // with at most one item per warp nothing is drawn (item_queue_release agrees)
+    const bool draw = DYN && total > nwarps;
+    for (unsigned int it = warp; it < total;) {
+        unsigned int next = DYN ? total : it + nwarps;
+        if (draw && rs.lane == 0)
+            next = draw_item(queue, nwarps);
+        stream_item(rs, ba, (int)it, eb);
+        it = draw ? __shfl_sync(kFull, next, 0) : next;
+    }
+}
+
+// End of a launch with the dynamic schedule: the last of `warps` warps to
+// finish puts the item counters back to zero for the next launch (every warp
+// has drawn its final item before it counts itself finished).
+__device__ __forceinline__ void item_queue_release(unsigned int *queue, const unsigned int nqueues,
+                                                   unsigned int *finished, const unsigned int warps)
 {
     if ((threadIdx.x & 31) == 0) {
-        const unsigned int warps = gridDim.x * gridDim.y * kWarpsPerBlock;
-        if (atomicAdd(queue + kMaxItemQueues, 1u) == warps - 1) {
-            for (unsigned t = 0; t < gridDim.y; t++)
+        if (atomicAdd(finished, 1u) == warps - 1) {
+            for (unsigned t = 0; t < nqueues; t++)
                 atomicExch(queue + t, 0u);
-            atomicExch(queue + kMaxItemQueues, 0u);
+            atomicExch(finished, 0u);
         }
     }
 }
 
-template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC_Y, int MINB = 1, bool DYN = false>
+// Launch of a dependent kernel may begin (its blocks wait for this grid's end
+// with pdl_wait): every block of these grids is resident when it says so.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB = 1, bool DYN = false>
 __global__ void __launch_bounds__(kThreads, MINB) rowblock_spmm_kernel(const __grid_constant__ BlockArgs ba,
                                                                        const typename ElemOf<TR>::T *__restrict__ X,
                                                                        int64_t ldx, TY *__restrict__ Y, int64_t ldy,
                                                                        int K, int accumulate)
 {
-    // the current batch of 32 (col, val) pairs of each warp, read back with
-    // one 8-byte shared-memory load per entry and lane group
-    __shared__ int2 s_ent[kWarpsPerBlock][32];
-    int2 *ent = s_ent[threadIdx.x >> 5];
+    __shared__ EntryBatch s_ent[kWarpsPerBlock];
+    pdl_launch_dependents();
     constexpr int W = LG * NV * TR::E;
     const int k0 = blockIdx.y * W;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    const int64_t total = ba.nseg + ba.ntask;
-    rowblock_items<TR, TY, LG, NV, UNROLL, VEC_Y, const BlockArgs, DYN>(
-        ba, (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5), nwarps, total, X, ldx, Y, ldy, K, accumulate,
-        k0, ent, 0, DYN ? ba.queue + blockIdx.y : nullptr);
-    if constexpr (DYN)
-        item_queue_release(ba.queue);
+    const unsigned int nwarps = gridDim.x * kWarpsPerBlock;
+    RowStream<TR, TY, LG, NV, UNROLL> rs;
+    rs.init(X, ldx, Y, ldy, K, k0, accumulate);
+    stream_items<RowStream<TR, TY, LG, NV, UNROLL>, DYN>(rs, ba, blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5),
+                                                         nwarps, s_ent[threadIdx.x >> 5],
+                                                         DYN ? ba.queue + blockIdx.y : nullptr);
+    if (DYN && (unsigned int)ba.nitem > nwarps)
+        item_queue_release(ba.queue, gridDim.y, ba.queue + kMaxItemQueues, nwarps * gridDim.y);
 }
 
 // The same schedule with the feature tiles one after another instead of side
 // by side (blockIdx.y): the grid sweeps every item of tile 0, then of tile 1,
 // ..., so the X columns being gathered at any moment are one tile wide.  Every
 // element's sum is the same chain of FMAs whichever tile width computes it
-// (one lane group per row: LG = 32).  A separate kernel, so that the default
-// one keeps its own register allocation.
+// (one lane group per row: LG = 32).
 template <typename TR, typename TY, int NV, int UNROLL, int MINB = 1>
 __global__ void __launch_bounds__(kThreads, MINB) rowblock_tiled_kernel(const __grid_constant__ BlockArgs ba,
                                                                         const typename ElemOf<TR>::T *__restrict__ X,
                                                                         int64_t ldx, TY *__restrict__ Y, int64_t ldy,
                                                                         int K, int accumulate)
 {
-    __shared__ int2 s_ent[kWarpsPerBlock][32];
-    int2 *ent = s_ent[threadIdx.x >> 5];
+    __shared__ EntryBatch s_ent[kWarpsPerBlock];
+    pdl_launch_dependents();
     constexpr int W = 32 * NV * TR::E;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    const int64_t total = ba.nseg + ba.ntask;
-    const int ntile = (K + W - 1) / W;
-    for (int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); w < total * ntile; w += nwarps) {
-        const int tile = (int)(w / total);
-        const int64_t it = w - (int64_t)tile * total;
-        rowblock_items<TR, TY, 32, NV, UNROLL, true>(ba, it, 1, it + 1, X, ldx, Y, ldy, K, accumulate, tile * W,
-                                                     ent);
+    const unsigned int nwarps = gridDim.x * kWarpsPerBlock;
+    // tile t starts where the last one's round robin over the warps ended
+    unsigned int warp = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    for (int k0 = 0; k0 < K; k0 += W) {
+        RowStream<TR, TY, 32, NV, UNROLL> rs;
+        rs.init(X, ldx, Y, ldy, K, k0, accumulate);
+        stream_items<RowStream<TR, TY, 32, NV, UNROLL>, false>(rs, ba, warp, nwarps, s_ent[threadIdx.x >> 5],
+                                                               nullptr);
+        warp = (warp + nwarps - (unsigned int)ba.nitem % nwarps) % nwarps;
     }
 }
 
@@ -587,78 +718,179 @@ __global__ void __launch_bounds__(kThreads) hub_combine_kernel(const int32_t *__
 }
 
 // Hub rows, 16-byte vector form (K a multiple of 4, ws rows 16-byte aligned):
-// one warp per (hub, 128-feature tile); every partial is read exactly once,
-// UNROLL partials in flight, and summed pairwise by a binary counter: partial
-// i is added to the running block sums of sizes 1, 2, 4, ... that its index's
-// trailing one bits close, so the sum is the same fixed binary tree for every
-// run.  The stack has one slot per tree level (at most 32).
-// One (hub, 128-feature tile) of the combine: partials ws[hub_seg[h] ..
-// hub_seg[h+1]) summed pairwise and written to output row hub_row[h].
-template <typename TY, int UNROLL>
-__device__ __forceinline__ void hub_combine_item(const int32_t *__restrict__ hub_row,
-                                                 const int64_t *__restrict__ hub_seg, const int64_t h, const int tile,
-                                                 const float *__restrict__ ws, const int64_t ld_ws, TY *__restrict__ Y,
-                                                 const int64_t ldy, const int K, const int accumulate)
+// a group of lc lanes (32, or the power of two that covers K / 4 below) owns one
+// (hub, 4 * lc-feature tile).  The m partials are added pairwise in the order of
+// a binary counter: partial i closes the running block sums of sizes 1, 2, 4,
+// ... that its index's trailing one bits name, and the open blocks at the end
+// are folded larger (earlier) first.  The counter is run kHubRadix partials at a
+// time, all their loads in flight and every running sum in a register: whole
+// blocks of kHubRadix are reduced to one value each in the workspace, blocks of
+// those to kHubRadix^2, and so on; then the open blocks of every power are
+// folded.  Hubs of kHubTeam or more partials are left to the end and each shared
+// by the whole block: one lane group alone walks 240 partials in 55 us, which
+// was the tail of the launch.
+constexpr int kHubRadixBits = 3, kHubRadix = 1 << kHubRadixBits;
+constexpr int kHubTeam = 32;
+constexpr int kHubList = 128;  // long hubs a block keeps for its end; more are walked alone
+
+// Counter over p[0 .. cnt) (stride ld floats, cnt <= kHubRadix).  FULL: tot =
+// the block's sum.  Otherwise folds the open blocks into tot (any: tot already
+// holds a sum).
+template <bool FULL>
+__device__ __forceinline__ void hub_counter(const float *p, const int64_t ld, const int cnt, float4 &tot, bool &any)
 {
-    const int lane = threadIdx.x & 31;
-    const int k = tile * 128 + lane * 4;
-    const bool kok = k < K;
-    const int64_t s0 = __ldg(hub_seg + h), m = __ldg(hub_seg + h + 1) - s0;
-    const float *wp = ws + s0 * ld_ws + k;
-    float4 stk[32];
-    for (int64_t i0 = 0; i0 < m; i0 += UNROLL) {
-        float4 v[UNROLL];
+    float4 v[kHubRadix];
 #pragma unroll
-        for (int u = 0; u < UNROLL; u++)
-            if (kok && i0 + u < m)
-                v[u] = __ldcg(reinterpret_cast<const float4 *>(wp + (i0 + u) * ld_ws));
-#pragma unroll
-        for (int u = 0; u < UNROLL; u++) {
-            const int64_t i = i0 + u;
-            if (i < m) {
-                float4 c = v[u];
-                int l = 0;
-                while ((i >> l) & 1) {
-                    const float4 a = stk[l];
-                    c = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w + c.w);
-                    l++;
-                }
-                stk[l] = c;
+    for (int i = 0; i < kHubRadix; i++, p += ld)
+        if (FULL || i < cnt)
+            v[i] = __ldcg(reinterpret_cast<const float4 *>(p));
+    auto add = [](float4 a, float4 c) {
+        return make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w + c.w);
+    };
+    // v[i] becomes the block that partial i closes; v[j] stays the open block ending at j
+    static_assert(kHubRadix == 8, "the blocks are spelled out");
+#define COLA_CLOSE(i, l)        \
+    if (FULL || (i) < cnt)      \
+        v[i] = add(v[(i) - (l)], v[i])
+    COLA_CLOSE(1, 1);
+    COLA_CLOSE(3, 1);
+    COLA_CLOSE(5, 1);
+    COLA_CLOSE(7, 1);
+    COLA_CLOSE(3, 2);
+    COLA_CLOSE(7, 2);
+    COLA_CLOSE(7, 4);
+#undef COLA_CLOSE
+    if (FULL) {
+        tot = v[kHubRadix - 1];
+        return;
+    }
+    auto pick = [](bool c, float4 a, float4 b) {
+        return make_float4(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z, c ? a.w : b.w);
+    };
+    auto fold = [&](float4 b) {
+        tot = any ? add(tot, b) : b;
+        any = true;
+    };
+    const bool c4 = cnt & 4, c2 = cnt & 2;
+    if (c4)
+        fold(v[3]);
+    if (c2)
+        fold(pick(c4, v[5], v[1]));
+    if (cnt & 1)
+        fold(pick(c4, pick(c2, v[6], v[4]), pick(c2, v[2], v[0])));
+}
+
+// One hub's tile of one output.
+template <typename TY>
+struct HubItem {
+    const int32_t *hub_row;
+    const int64_t *hub_seg;
+    int64_t h;
+    int tile;
+    float *ws;
+    int64_t ld_ws;
+    TY *Y;
+    int64_t ldy;
+    int K;
+    __device__ __forceinline__ int partials() const { return (int)(__ldg(hub_seg + h + 1) - __ldg(hub_seg + h)); }
+};
+
+// One item by `teams` lane groups of which this is number `team`: the m partials
+// at wp (rows of ld floats; this lane's 4 features) to y.  One copy of the code
+// for both kinds of call.  A lane re-reads the sums of its own features only;
+// with several teams the block waits between powers.
+template <typename TY>
+__device__ __noinline__ void hub_combine_item(float *wp, const int64_t ld, const int m, TY *y, const bool kok,
+                                              const int accumulate, const int team, const int teams)
+{
+    float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool any = false;
+    // whole blocks of kHubRadix^1, ^2, ... partials: each block's sum over its first partial
+    int power = 0;  // log2 of the partials per element
+    for (int n = m >> kHubRadixBits; n > 0; n >>= kHubRadixBits, power += kHubRadixBits) {
+        if (kok)
+#pragma unroll 1
+            for (int c = team; c < n; c += teams) {
+                float *p = wp + ((int64_t)c << (power + kHubRadixBits)) * ld;
+                float4 b;
+                hub_counter<true>(p, ld << power, kHubRadix, b, any);
+                __stcg(reinterpret_cast<float4 *>(p), b);
+            }
+        if (teams > 1)
+            __syncthreads();
+    }
+    if (team != 0 || !kok)
+        return;
+    // the open blocks, larger powers (earlier partials) first
+    int base = 0;
+#pragma unroll 1
+    for (; power >= 0; power -= kHubRadixBits) {
+        const int cnt = (m - base) >> power;
+        if (cnt > 0)
+            hub_counter<false>(wp + base * ld, ld << power, cnt, tot, any);
+        base += cnt << power;
+    }
+    const float r[4] = {tot.x, tot.y, tot.z, tot.w};
+    store_out<TY, 4, true>(y, r, accumulate != 0);
+}
+
+// Lanes per (hub, tile) of the combine and tiles per hub.
+__host__ __device__ inline int hub_lanes(int K) { return K > 64 ? 32 : K > 32 ? 16 : K > 16 ? 8 : 4; }
+__host__ __device__ inline int hub_tiles(int K) { return (K + 127) / 128; }
+
+// Combine items [0, total) with `lc` lanes each; find(w) names item w.
+// Neighbouring items (in R-MAT order: hubs of like length) go to different
+// blocks.
+template <typename TY, typename FIND>
+__device__ __forceinline__ void hub_combine_all(const int64_t total, const int lc, const int accumulate, FIND find)
+{
+    __shared__ int64_t s_big[kHubList];
+    __shared__ int s_nbig;
+    if (threadIdx.x == 0)
+        s_nbig = 0;
+    __syncthreads();
+    const int groups = kThreads / lc, grp = threadIdx.x / lc, gl = threadIdx.x % lc;
+    const unsigned int mask = lc == 32 ? kFull : ((1u << lc) - 1u) << ((threadIdx.x & 31) / lc * lc);
+    auto combine = [&](const HubItem<TY> &it, int m, int team, int teams) {
+        const int k = it.tile * 128 + gl * 4;
+        hub_combine_item<TY>(it.ws + __ldg(it.hub_seg + it.h) * it.ld_ws + k, it.ld_ws, m,
+                             it.Y + (int64_t)__ldg(it.hub_row + it.h) * it.ldy + k, k < it.K, accumulate, team, teams);
+    };
+    for (int64_t w = (int64_t)grp * gridDim.x + blockIdx.x; w < total; w += (int64_t)gridDim.x * groups) {
+        const HubItem<TY> it = find(w);
+        const int m = it.partials();
+        if (m >= kHubTeam) {
+            int at = 0;
+            if (gl == 0)
+                at = atomicAdd(&s_nbig, 1);
+            at = __shfl_sync(mask, at, 0, lc);
+            if (at < kHubList) {
+                if (gl == 0)
+                    s_big[at] = w;
+                continue;
             }
         }
+        combine(it, m, 0, 1);
     }
-    // fold the open block sums, larger (earlier) blocks first
-    float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
-    bool first = true;
-    for (int l = 31; l >= 0; l--)
-        if ((m >> l) & 1) {
-            const float4 a = stk[l];
-            tot = first ? a : make_float4(tot.x + a.x, tot.y + a.y, tot.z + a.z, tot.w + a.w);
-            first = false;
-        }
-    if (kok) {
-        const float r[4] = {tot.x, tot.y, tot.z, tot.w};
-        store_out<TY, 4, true>(Y + (int64_t)__ldg(hub_row + h) * ldy + k, r, accumulate != 0);
+    __syncthreads();
+    const int nbig = min(s_nbig, kHubList);
+    for (int q = 0; q < nbig; q++) {
+        const HubItem<TY> it = find(s_big[q]);
+        combine(it, it.partials(), grp, groups);
     }
 }
 
-// Hub rows, 16-byte vector form (K a multiple of 4, ws rows 16-byte aligned):
-// one warp per (hub, 128-feature tile); every partial is read exactly once,
-// UNROLL partials in flight, and summed pairwise by a binary counter: partial
-// i is added to the running block sums of sizes 1, 2, 4, ... that its index's
-// trailing one bits close, so the sum is the same fixed binary tree for every
-// run.  The stack has one slot per tree level (at most 32).
-template <typename TY, int UNROLL>
-__global__ void __launch_bounds__(kThreads) hub_combine_vec_kernel(const int32_t *__restrict__ hub_row,
+template <typename TY>
+__global__ void __launch_bounds__(kThreads, 3) hub_combine_vec_kernel(const int32_t *__restrict__ hub_row,
                                                                   const int64_t *__restrict__ hub_seg, int64_t nhub,
-                                                                  const float *__restrict__ ws, int64_t ld_ws,
-                                                                  TY *__restrict__ Y, int64_t ldy, int K,
-                                                                  int accumulate)
+                                                                  float *ws, int64_t ld_ws, TY *__restrict__ Y,
+                                                                  int64_t ldy, int K, int accumulate)
 {
-    const int tiles = (K + 127) / 128;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    for (int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); w < nhub * tiles; w += nwarps)
-        hub_combine_item<TY, UNROLL>(hub_row, hub_seg, w / tiles, (int)(w % tiles), ws, ld_ws, Y, ldy, K, accumulate);
+    pdl_wait();  // the partials
+    const int tiles = hub_tiles(K);
+    hub_combine_all<TY>(nhub * tiles, hub_lanes(K), accumulate, [&](int64_t w) {
+        return HubItem<TY>{hub_row, hub_seg, w / tiles, (int)(w % tiles), ws, ld_ws, Y, ldy, K};
+    });
 }
 
 }  // namespace dev

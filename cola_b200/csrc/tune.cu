@@ -52,7 +52,6 @@ std::vector<Cand> rows_candidates(cola_dtype xdt, int K)
             c.push_back({kt, 2, 0, 0});
             for (int mb : {3, 4})
                 c.push_back({kt, 4, mb, 0});
-            c.push_back({kt, 6, 0, 0});
             c.push_back({kt, 8, 0, 0});
         } else if (V == 64) {
             c.push_back({kt, 2, 0, 0});
