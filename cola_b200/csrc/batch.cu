@@ -33,6 +33,8 @@ struct cola_batch {
     std::vector<BatchGraph> h_desc;  // graphs that run in the batched launch
     BatchGraph *d_desc = nullptr;
     size_t d_desc_bytes = 0;
+    float *d_ws = nullptr;  // hub partials of the batched graphs
+    size_t d_ws_bytes = 0;
     cola::BatchLaunch launch = {};  // groups and totals of h_desc
     int64_t total_items = 0, total_hub = 0;
     struct Solo {  // graphs that run through cola_spmm (scalar path or K > 32 vectors)
@@ -68,6 +70,7 @@ static void batch_release(cola_batch *b)
     if (b->cgraph)
         cudaGraphDestroy(b->cgraph);
     cudaFree(b->d_desc);
+    cudaFree(b->d_ws);
     if (b->own_graphs)
         for (cola_graph *g : b->graphs)
             graph_release(g);
@@ -335,6 +338,8 @@ cola_status cola_batch_bind(cola_batch *b, const void *const *X, const int64_t *
     b->solo.clear();
     b->total_items = 0;
     b->total_hub = 0;
+    std::vector<size_t> ws_off;  // of each batched graph's hub workspace
+    size_t ws_floats = 0;
     for (size_t i = 0; i < b->graphs.size(); i++) {
         cola_graph *g = b->graphs[i];
         COLA_REQUIRE(K[i] >= 1 && ldx[i] >= K[i] && ldy[i] >= K[i] && (g->N == 0 || (X[i] && Y[i])),
@@ -342,24 +347,24 @@ cola_status cola_batch_bind(cola_batch *b, const void *const *X, const int64_t *
                      (long long)ldx[i], (long long)ldy[i]);
         if (g->N == 0)
             continue;
-        if (g->nseg > 0)
-            COLA_TRY(ensure(reinterpret_cast<void *&>(g->ws_hub), g->ws_hub_bytes,
-                            (size_t)g->nseg * K[i] * sizeof(float)));
-        // a graph that is in the batch twice has one hub workspace: its second
-        // product runs after the batch
-        bool again = false;
-        for (size_t j = 0; j < i && g->nseg > 0 && !again; j++)
-            again = b->graphs[j] == g;
-        const bool vec = vec_ok_rows(xdt, X[i], ldx[i], ydt, Y[i], ldy[i], K[i]) && aligned16(g->ws_hub);
-        if (!vec || again) {
+        if (!vec_ok_rows(xdt, X[i], ldx[i], ydt, Y[i], ldy[i], K[i])) {
             b->solo.push_back({(int)i, X[i], ldx[i], Y[i], ldy[i], K[i]});
             continue;
         }
         BatchGraph d;
-        fill_batch_graph(d, g, X[i], ldx[i], Y[i], ldy[i], K[i], xdt, g->ws_hub);
+        // the batch's own hub workspace: offsets here, addresses once it is sized
+        fill_batch_graph(d, g, X[i], ldx[i], Y[i], ldy[i], K[i], xdt, nullptr);
+        ws_off.push_back(ws_floats);
+        ws_floats += (size_t)g->nseg * K[i];
         b->total_items += g->nseg + g->ntask;
         b->h_desc.push_back(d);
     }
+    void *ws = b->d_ws;
+    const cola_status ws_ok = ensure(ws, b->d_ws_bytes, ws_floats * sizeof(float));
+    b->d_ws = static_cast<float *>(ws);
+    COLA_TRY(ws_ok);
+    for (size_t i = 0; i < b->h_desc.size(); i++)
+        b->h_desc[i].ba.ws = b->d_ws + ws_off[i];
     COLA_TRY(build_groups(b->h_desc.data(), (int)b->h_desc.size(), b->launch));
     b->total_hub = b->launch.total_hub;
     const size_t qoff = batch_queue_offset(b->h_desc.size() * sizeof(BatchGraph));
@@ -439,7 +444,7 @@ cola_status cola_batch_get_info(const cola_batch *b, cola_batch_info *o)
         o->nnz += g->nnz_l + g->nnz_r;
         o->device_bytes += (int64_t)(g->dbytes + g->ws_hub_bytes);
     }
-    o->device_bytes += (int64_t)b->d_desc_bytes;
+    o->device_bytes += (int64_t)(b->d_desc_bytes + b->d_ws_bytes);
     o->unroll = b->unroll;
     o->grid_pct = b->grid_pct;
     o->blocks_per_sm = b->blocks_per_sm;

@@ -77,7 +77,8 @@ void host_pipe_release(HostPipe *p);
 
 struct cola_graph {
     int device = 0;
-    int32_t N = 0, P = 0, npp = 0, gs = 0, nstages = 1, if_split = 1;
+    int32_t N = 0, NX = 0;  // rows of Y, rows of X (columns of the matrix)
+    int32_t P = 0, npp = 0, gs = 0, nstages = 1, if_split = 1;
     int64_t nnz_l = 0, nnz_r = 0, lchunks = 0, rchunks = 0, rcols = 0;
     void *dmem = nullptr;
     size_t dbytes = 0;
@@ -127,6 +128,8 @@ struct cola_graph {
     // in dmem, zero between launches
     unsigned int *item_queue = nullptr;
     size_t ws_hub_bytes = 0;
+    void *x_pad = nullptr;  // X with padded rows (widths no vector divides)
+    size_t x_pad_bytes = 0;
     cola::HostPipe *host_pipe = nullptr;  // created by the first cola_spmm_host call
 };
 

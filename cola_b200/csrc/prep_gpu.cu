@@ -1026,6 +1026,7 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     COLA_REQUIRE(g, COLA_ERROR_OUT_OF_MEMORY, "%s: host allocation failed", who);
     COLA_CUDA(cudaGetDevice(&g->device));
     g->N = N;
+    g->NX = NC;
     g->P = nparts;
     g->npp = (int32_t)npp;
     g->gs = nparts;

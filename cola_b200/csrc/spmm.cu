@@ -390,6 +390,53 @@ static cola_status launch_block_t(const dev::BlockArgs &ba, const RowsLaunch &a,
     return COLA_SUCCESS;
 }
 
+// Element-wise output (VEC_Y false): the default geometry of the width.
+template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB>
+static cola_status launch_block_odd_t(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
+{
+    using T = typename dev::ElemOf<TR>::T;
+    constexpr int W = LG * NV * TR::E;
+    const int64_t ntile = (a.K + W - 1) / W;
+    const bool dyn = ba.queue && ntile <= dev::kMaxItemQueues;
+    auto fn = dyn ? dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, true, false>
+                  : dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, false, false>;
+    t_launches++;
+    COLA_CUDA(launch_kernel(fn, (unsigned)grid_for((const void *)fn, ba.nitem), (unsigned)ntile, false, st, ba,
+                            static_cast<const T *>(a.X), a.ldx, static_cast<TY *>(a.Y), a.ldy, a.K, a.accumulate));
+    return COLA_SUCCESS;
+}
+
+template <typename TR, typename TY>
+static cola_status launch_block_odd_geo(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
+{
+    const int V = (a.K + TR::E - 1) / TR::E;
+    if (V <= 1)
+        return launch_block_odd_t<TR, TY, 1, 1, 1, 4>(ba, a, st);
+    if (V <= 2)
+        return launch_block_odd_t<TR, TY, 2, 1, 2, 4>(ba, a, st);
+    if (V <= 4)
+        return launch_block_odd_t<TR, TY, 4, 1, 4, 4>(ba, a, st);
+    if (V <= 8)
+        return launch_block_odd_t<TR, TY, 8, 1, 4, 4>(ba, a, st);
+    if (V <= 16)
+        return launch_block_odd_t<TR, TY, 16, 1, 4, 4>(ba, a, st);
+    if (V <= 32)
+        return launch_block_odd_t<TR, TY, 32, 1, 4, 4>(ba, a, st);
+    return launch_block_odd_t<TR, TY, 32, 2, 4, 3>(ba, a, st);
+}
+
+static cola_status launch_block_odd(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
+{
+    if (ba.nitem <= 0)
+        return COLA_SUCCESS;
+    using BF = __nv_bfloat16;
+    if (a.xdt == COLA_FLOAT32)
+        return a.ydt == COLA_FLOAT32 ? launch_block_odd_geo<dev::VecTraits<float>, float>(ba, a, st)
+                                     : launch_block_odd_geo<dev::VecTraits<float>, BF>(ba, a, st);
+    return a.ydt == COLA_FLOAT32 ? launch_block_odd_geo<dev::VecTraits<BF>, float>(ba, a, st)
+                                 : launch_block_odd_geo<dev::VecTraits<BF>, BF>(ba, a, st);
+}
+
 // Narrow passes (a full warp on a 64- or 128-feature tile, 8 or 4 bytes per
 // lane): loads in flight 4 or 8, resident blocks per SM 4, 6 or 8.
 template <typename TR, typename TY>
@@ -505,6 +552,51 @@ bool vec_ok_rows(cola_dtype xdt, const void *X, int64_t ldx, cola_dtype ydt, con
     if (ldy % E || ((uintptr_t)Y % (uintptr_t)(E * ysz)) != 0)
         return false;
     return true;
+}
+
+// X as the vector form reads it: itself where its rows are whole aligned
+// vectors, else a padded copy in the graph's workspace (x_ok false: neither).
+// The copy is two passes over X against one over X per entry of a row, so it is
+// made from 2 entries a row on; not while the stream is being captured with too
+// small a workspace (allocating would break the capture), nor when the device
+// has no room for it.  The scalar kernel remains for those calls.  K = 33 FP32,
+// 150 K rows, 2.4 M entries: 185 -> 73 us, K = 74 BF16 209 -> 100, K = 301 FP32
+// 717 -> 337, K = 33 at 3 entries a row 86 -> 42.
+static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool &x_ok, cudaStream_t st)
+{
+    const int E = a.xdt == COLA_FLOAT32 ? 4 : 8, esz = 16 / E;
+    x_ok = a.K % E == 0 && a.ldx % E == 0 && a.ldx <= INT32_MAX / esz && aligned16(a.X);
+    if (x_ok || g->nnz_l + g->nnz_r < 2 * (int64_t)g->NX)
+        return COLA_SUCCESS;
+    const int64_t nvec = (a.K + E - 1) / E;
+    const size_t bytes = (size_t)g->NX * nvec * 16;
+    if (g->x_pad_bytes < bytes) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        COLA_CUDA(cudaStreamIsCapturing(st, &cap));
+        if (cap != cudaStreamCaptureStatusNone)
+            return COLA_SUCCESS;
+        if (ensure(g->x_pad, g->x_pad_bytes, bytes) != COLA_SUCCESS) {
+            cudaGetLastError();
+            clear_error();
+            return COLA_SUCCESS;
+        }
+    }
+    const int64_t total = g->NX * nvec;
+    const unsigned blocks = (unsigned)std::min<int64_t>((total + dev::kThreads - 1) / dev::kThreads,
+                                                        (int64_t)sm_count() * 32);
+    t_launches++;
+    if (a.xdt == COLA_FLOAT32)
+        dev::pad_rows_kernel<float><<<blocks, dev::kThreads, 0, st>>>(
+            static_cast<const float *>(a.X), a.ldx, static_cast<float *>(g->x_pad), (int)nvec, total, a.K);
+    else
+        dev::pad_rows_kernel<__nv_bfloat16><<<blocks, dev::kThreads, 0, st>>>(
+            static_cast<const __nv_bfloat16 *>(a.X), a.ldx, static_cast<__nv_bfloat16 *>(g->x_pad), (int)nvec, total,
+            a.K);
+    COLA_CUDA(cudaGetLastError());
+    a.X = g->x_pad;
+    a.ldx = nvec * E;
+    x_ok = true;
+    return COLA_SUCCESS;
 }
 
 static PartDesc part_desc_zero()
@@ -735,6 +827,7 @@ void graph_release(cola_graph *g)
     cudaFree(g->stage_buf);
     cudaFree(g->ws);
     cudaFree(g->ws_hub);
+    cudaFree(g->x_pad);
     host_pipe_release(g->host_pipe);
     cudaSetDevice(cur);
     delete g;
@@ -768,7 +861,7 @@ cola_status graph_upload(const cola_partition_set *ps, const cola_upload_opts *o
         COLA_TRY(validate_partition(*ps, ph));
     std::unique_ptr<cola_graph, void (*)(cola_graph *)> g(new cola_graph(), graph_release);
     COLA_CUDA(cudaGetDevice(&g->device));
-    g->N = ps->num_nodes;
+    g->N = g->NX = ps->num_nodes;
     g->P = P;
     g->npp = ps->npp;
     g->gs = gs;
@@ -1085,7 +1178,8 @@ cola_status cola_graph_get_info(const cola_graph *g, cola_graph_info *o)
     o->local_chunks = g->lchunks;
     o->remote_chunks = g->rchunks;
     o->remote_cols = g->rcols;
-    o->device_bytes = (int64_t)(g->dbytes + g->ppl_bytes + g->stage_bytes + g->ws_bytes + g->ws_hub_bytes);
+    o->device_bytes = (int64_t)(g->dbytes + g->ppl_bytes + g->stage_bytes + g->ws_bytes + g->ws_hub_bytes +
+                                  g->x_pad_bytes);
     o->hub_rows = g->nhub;
     o->hub_segments = g->nseg;
     o->row_tasks = g->ntask;
@@ -1180,8 +1274,11 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
 
     if (schedule == COLA_SCHEDULE_ROWS) {
         // one writer per output row: Y written directly in its own dtype
+        // rows of the hub workspace are whole vectors of X
+        const int64_t E = xdt == COLA_FLOAT32 ? 4 : 8, ldw = (K + E - 1) / E * E;
         if (g->nseg > 0)
-            COLA_TRY(ensure(reinterpret_cast<void *&>(g->ws_hub), g->ws_hub_bytes, (size_t)g->nseg * K * sizeof(float)));
+            COLA_TRY(ensure(reinterpret_cast<void *&>(g->ws_hub), g->ws_hub_bytes,
+                            (size_t)g->nseg * ldw * sizeof(float)));
         RowsLaunch a;
         a.ra.rowptr = g->rv_ptr;
         a.ra.col = g->rv_col;
@@ -1193,7 +1290,7 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         a.ra.nseg = g->nseg;
         a.ra.seg_len = g->hub_segment;
         a.ra.ws = g->ws_hub;
-        a.ra.ld_ws = K;
+        a.ra.ld_ws = ldw;
         a.X = X;
         a.ldx = ldx;
         a.Y = Y;
@@ -1206,32 +1303,37 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         a.unroll = opts ? opts->unroll : 0;
         a.min_blocks = opts ? opts->min_blocks : 0;
         a.k_tile = opts ? opts->k_tile : 0;
-        if (a.vec) {
-            COLA_TRY(launch_block(block_args(g, g->ws_hub, K), a, st));
-        } else {
+        bool x_ok = a.vec;
+        if (!a.vec)
+            COLA_TRY(pad_x(g, a, x_ok, st));
+        if (a.vec)
+            COLA_TRY(launch_block(block_args(g, g->ws_hub, ldw), a, st));
+        else if (x_ok)
+            COLA_TRY(launch_block_odd(block_args(g, g->ws_hub, ldw), a, st));
+        else
             COLA_TRY(launch_rows(a, st));
-        }
-        if (g->nhub > 0 && a.vec && K % 4 == 0 && ldy % 4 == 0 &&
-            aligned16(g->ws_hub) && ((uintptr_t)Y % (ydt == COLA_FLOAT32 ? 16 : 8)) == 0) {
+        if (g->nhub > 0 && x_ok) {
             const unsigned blocks = hub_blocks(g->nhub * dev::hub_tiles(K), dev::hub_lanes(K));
             t_launches++;
-            if (ydt == COLA_FLOAT32)
-                COLA_CUDA(launch_kernel(dev::hub_combine_vec_kernel<float>, blocks, 1, true, st, g->hub_row,
-                                        g->hub_seg, g->nhub, g->ws_hub, K, static_cast<float *>(Y), ldy, K,
-                                        accumulate));
-            else
-                COLA_CUDA(launch_kernel(dev::hub_combine_vec_kernel<__nv_bfloat16>, blocks, 1, true, st, g->hub_row,
-                                        g->hub_seg, g->nhub, g->ws_hub, K, static_cast<__nv_bfloat16 *>(Y), ldy, K,
-                                        accumulate));
+            using BF = __nv_bfloat16;
+            if (ydt == COLA_FLOAT32) {
+                auto fn = a.vec ? dev::hub_combine_vec_kernel<float, true> : dev::hub_combine_vec_kernel<float, false>;
+                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw,
+                                        static_cast<float *>(Y), ldy, K, accumulate));
+            } else {
+                auto fn = a.vec ? dev::hub_combine_vec_kernel<BF, true> : dev::hub_combine_vec_kernel<BF, false>;
+                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw,
+                                        static_cast<BF *>(Y), ldy, K, accumulate));
+            }
         } else if (g->nhub > 0) {
             const int64_t blocks = (g->nhub + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock;
             t_launches++;
             if (ydt == COLA_FLOAT32)
                 dev::hub_combine_kernel<float><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, K, static_cast<float *>(Y), ldy, K, accumulate);
+                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw, static_cast<float *>(Y), ldy, K, accumulate);
             else
                 dev::hub_combine_kernel<__nv_bfloat16><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, K, static_cast<__nv_bfloat16 *>(Y), ldy, K,
+                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw, static_cast<__nv_bfloat16 *>(Y), ldy, K,
                     accumulate);
             COLA_CUDA(cudaGetLastError());
         }

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kThreads, 3) batch_hub_combine_kernel(const Ba
 {
     pdl_wait();  // the partials
     int gi = 0;
-    hub_combine_all<TY>(total, lanes, accumulate, [&](int64_t w) {
+    hub_combine_all<TY, true>(total, lanes, accumulate, [&](int64_t w) {
         if (w < gs[gi].hub0)
             gi = 0;
         while (gi + 1 < ng && w >= gs[gi + 1].hub0)

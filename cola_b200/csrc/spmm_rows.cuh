@@ -11,8 +11,6 @@
 // a second kernel adds each hub's partials pairwise (a binary tree in fixed
 // order) and writes the row.
 #pragma once
-#include <type_traits>
-
 #include "spmm_kernels.cuh"
 
 namespace cola {
@@ -93,6 +91,19 @@ template <>
 __device__ __forceinline__ void store_out<__nv_bfloat16, 1, false>(__nv_bfloat16 *p, const float (&a)[1], bool)
 {
     *p = __float2bfloat16_rn(a[0]);
+}
+
+// The first `left` (at most E) of a lane's values, one element at a time: an
+// output whose rows are not vector-aligned or end inside a vector.
+template <typename TY, int E>
+__device__ __forceinline__ void store_some(TY *p, const float (&a)[E], bool accumulate, int left)
+{
+#pragma unroll
+    for (int q = 0; q < E; q++)
+        if (q < left) {
+            const float v[1] = {a[q]};
+            store_out<TY, 1, false>(p + q, v, accumulate);
+        }
 }
 
 // Hub segment table: segment s covers entries [beg[s], min(beg[s]+seg_len,
@@ -321,7 +332,9 @@ __device__ __forceinline__ int lane_id()
 // BF16 206 -> 126 us, K = 32 FP32 on 16 K rows 23 -> 14 us.  Slower: 8 rows in
 // flight at 3 blocks (1.10 ms), 2 at 5 or 6 (1.35), the next row's load issued
 // as each row is added (1.64).
-template <typename TR, typename TY, int LG, int NV, int UNROLL>
+// VEC_Y: rows of Y are written in vectors; else (their start is not aligned or K
+// ends inside a vector of X) element by element, X still read in vectors.
+template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC_Y = true>
 struct RowStream {
     using T = typename ElemOf<TR>::T;
     using raw_t = typename TR::raw_t;
@@ -337,12 +350,15 @@ struct RowStream {
     TY *Y;
     int64_t ldy;
     int koff;  // the lane's first feature
+    int K;
     int lane, g, gl;
     bool kok[NV];
     bool accumulate;
+    bool to_ws;  // the current item's row goes to the workspace
 
-    __device__ __forceinline__ void init(const T *X, int64_t ldx_, TY *Y_, int64_t ldy_, int K, int k0, int acc_)
+    __device__ __forceinline__ void init(const T *X, int64_t ldx_, TY *Y_, int64_t ldy_, int K_, int k0, int acc_)
     {
+        K = K_;
         lane = lane_id();
         g = lane / LG;
         gl = lane % LG;
@@ -366,6 +382,18 @@ struct RowStream {
                 acc[j][q] = make_float2(0.f, 0.f);
     }
 
+    // N values of a row of Y or, always in vectors, of the workspace.
+    template <typename TO, int N>
+    __device__ __forceinline__ void put(TO *p, const float (&a)[N], bool add, int left) const
+    {
+        if constexpr (VEC_Y)
+            store_out<TO, N, (N > 1)>(p, a, add);
+        else if (to_ws)
+            store_out<TO, N, (N > 1)>(p, a, false);
+        else
+            store_some<TO, N>(p, a, add, left);
+    }
+
     // The warp's sums to one row of Y or of the workspace (p: the lane's first
     // feature in that row); clears them.
     template <typename TO>
@@ -381,7 +409,7 @@ struct RowStream {
                     a[2 * q + 1] = acc[j][q].y;
                 }
                 if (kok[j])
-                    store_out<TO, E, true>(p + j * LG * E, a, add);
+                    put(p + j * LG * E, a, add, K - koff - j * LG * E);
             }
         } else {
             float v[E];
@@ -416,7 +444,7 @@ struct RowStream {
 #pragma unroll
                 for (int q = 0; q < EO; q++)
                     a[q] = v[q];
-                store_out<TO, EO, (EO > 1)>(p + f, a, add);
+                put(p + f, a, add, K - koff - f);
             }
         }
         clear();
@@ -542,6 +570,7 @@ __device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const i
 {
     const int lane = rs.lane;
     const bool seg = it < ba.nseg;
+    rs.to_ws = seg;
     const WorkItem w = load_item(ba.item + it);
     int64_t pos = w.beg + lane;
     int left = w.n;
@@ -578,7 +607,7 @@ __device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const i
         rs.write_row(ba.ws + (int64_t)it * ba.ld_ws + rs.koff, false);
     // this item's share of the empty rows, G rows at a time
     if (ba.nempty > 0 && !rs.accumulate) {
-        using TY = typename std::remove_pointer<decltype(rs.Y)>::type;
+        rs.to_ws = false;
         const int64_t z0 = (int64_t)it * ba.empty_share;
         const int zn = (int)min((int64_t)ba.empty_share, ba.nempty - z0);
         for (int i = rs.g; i < zn; i += RS::G) {
@@ -587,7 +616,8 @@ __device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const i
 #pragma unroll
             for (int j = 0; j < RS::NVEC; j++)
                 if (rs.kok[j])
-                    store_out<TY, RS::E, true>(rs.Y + (int64_t)row * rs.ldy + rs.koff + j * RS::LANES * RS::E, z, false);
+                    rs.put(rs.Y + (int64_t)row * rs.ldy + rs.koff + j * RS::LANES * RS::E, z, false,
+                           rs.K - rs.koff - j * RS::LANES * RS::E);
         }
         __syncwarp();
     }
@@ -639,7 +669,7 @@ __device__ __forceinline__ void item_queue_release(unsigned int *queue, const un
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB = 1, bool DYN = false>
+template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB = 1, bool DYN = false, bool VEC_Y = true>
 __global__ void __launch_bounds__(kThreads, MINB) rowblock_spmm_kernel(const __grid_constant__ BlockArgs ba,
                                                                        const typename ElemOf<TR>::T *__restrict__ X,
                                                                        int64_t ldx, TY *__restrict__ Y, int64_t ldy,
@@ -650,9 +680,9 @@ __global__ void __launch_bounds__(kThreads, MINB) rowblock_spmm_kernel(const __g
     constexpr int W = LG * NV * TR::E;
     const int k0 = blockIdx.y * W;
     const unsigned int nwarps = gridDim.x * kWarpsPerBlock;
-    RowStream<TR, TY, LG, NV, UNROLL> rs;
+    RowStream<TR, TY, LG, NV, UNROLL, VEC_Y> rs;
     rs.init(X, ldx, Y, ldy, K, k0, accumulate);
-    stream_items<RowStream<TR, TY, LG, NV, UNROLL>, DYN>(rs, ba, blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5),
+    stream_items<RowStream<TR, TY, LG, NV, UNROLL, VEC_Y>, DYN>(rs, ba, blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5),
                                                          nwarps, s_ent[threadIdx.x >> 5],
                                                          DYN ? ba.queue + blockIdx.y : nullptr);
     if (DYN && (unsigned int)ba.nitem > nwarps)
@@ -717,7 +747,7 @@ __global__ void __launch_bounds__(kThreads) hub_combine_kernel(const int32_t *__
     }
 }
 
-// Hub rows, 16-byte vector form (K a multiple of 4, ws rows 16-byte aligned):
+// Hub rows, 16-byte vector form (ws rows 16-byte aligned, of whole vectors):
 // a group of lc lanes (32, or the power of two that covers K / 4 below) owns one
 // (hub, 4 * lc-feature tile).  The m partials are added pairwise in the order of
 // a binary counter: partial i closes the running block sums of sizes 1, 2, 4,
@@ -799,10 +829,11 @@ struct HubItem {
 // at wp (rows of ld floats; this lane's 4 features) to y.  One copy of the code
 // for both kinds of call.  A lane re-reads the sums of its own features only;
 // with several teams the block waits between powers.
-template <typename TY>
-__device__ __noinline__ void hub_combine_item(float *wp, const int64_t ld, const int m, TY *y, const bool kok,
+template <typename TY, bool VEC_Y>
+__device__ __noinline__ void hub_combine_item(float *wp, const int64_t ld, const int m, TY *y, const int left,
                                               const int accumulate, const int team, const int teams)
 {
+    const bool kok = left > 0;
     float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
     bool any = false;
     // whole blocks of kHubRadix^1, ^2, ... partials: each block's sum over its first partial
@@ -831,7 +862,10 @@ __device__ __noinline__ void hub_combine_item(float *wp, const int64_t ld, const
         base += cnt << power;
     }
     const float r[4] = {tot.x, tot.y, tot.z, tot.w};
-    store_out<TY, 4, true>(y, r, accumulate != 0);
+    if constexpr (VEC_Y)
+        store_out<TY, 4, true>(y, r, accumulate != 0);
+    else
+        store_some<TY, 4>(y, r, accumulate != 0, left);
 }
 
 // Lanes per (hub, tile) of the combine and tiles per hub.
@@ -841,7 +875,7 @@ __host__ __device__ inline int hub_tiles(int K) { return (K + 127) / 128; }
 // Combine items [0, total) with `lc` lanes each; find(w) names item w.
 // Neighbouring items (in R-MAT order: hubs of like length) go to different
 // blocks.
-template <typename TY, typename FIND>
+template <typename TY, bool VEC_Y, typename FIND>
 __device__ __forceinline__ void hub_combine_all(const int64_t total, const int lc, const int accumulate, FIND find)
 {
     __shared__ int64_t s_big[kHubList];
@@ -853,8 +887,8 @@ __device__ __forceinline__ void hub_combine_all(const int64_t total, const int l
     const unsigned int mask = lc == 32 ? kFull : ((1u << lc) - 1u) << ((threadIdx.x & 31) / lc * lc);
     auto combine = [&](const HubItem<TY> &it, int m, int team, int teams) {
         const int k = it.tile * 128 + gl * 4;
-        hub_combine_item<TY>(it.ws + __ldg(it.hub_seg + it.h) * it.ld_ws + k, it.ld_ws, m,
-                             it.Y + (int64_t)__ldg(it.hub_row + it.h) * it.ldy + k, k < it.K, accumulate, team, teams);
+        hub_combine_item<TY, VEC_Y>(it.ws + __ldg(it.hub_seg + it.h) * it.ld_ws + k, it.ld_ws, m,
+                             it.Y + (int64_t)__ldg(it.hub_row + it.h) * it.ldy + k, it.K - k, accumulate, team, teams);
     };
     for (int64_t w = (int64_t)grp * gridDim.x + blockIdx.x; w < total; w += (int64_t)gridDim.x * groups) {
         const HubItem<TY> it = find(w);
@@ -880,7 +914,7 @@ __device__ __forceinline__ void hub_combine_all(const int64_t total, const int l
     }
 }
 
-template <typename TY>
+template <typename TY, bool VEC_Y>
 __global__ void __launch_bounds__(kThreads, 3) hub_combine_vec_kernel(const int32_t *__restrict__ hub_row,
                                                                   const int64_t *__restrict__ hub_seg, int64_t nhub,
                                                                   float *ws, int64_t ld_ws, TY *__restrict__ Y,
@@ -888,9 +922,28 @@ __global__ void __launch_bounds__(kThreads, 3) hub_combine_vec_kernel(const int3
 {
     pdl_wait();  // the partials
     const int tiles = hub_tiles(K);
-    hub_combine_all<TY>(nhub * tiles, hub_lanes(K), accumulate, [&](int64_t w) {
+    hub_combine_all<TY, VEC_Y>(nhub * tiles, hub_lanes(K), accumulate, [&](int64_t w) {
         return HubItem<TY>{hub_row, hub_seg, w / tiles, (int)(w % tiles), ws, ld_ws, Y, ldy, K};
     });
+}
+
+// X with every row padded to whole 16-byte vectors (zeros), for the vector form
+// when K or the rows' alignment does not allow it: one thread per vector.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) pad_rows_kernel(const T *__restrict__ X, int64_t ldx, T *__restrict__ P,
+                                                           int nvec, int64_t total, int K)
+{
+    constexpr int E = 16 / sizeof(T);
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kThreads) {
+        const int64_t r = i / nvec;
+        const int k = (int)(i - r * nvec) * E;
+        const T *p = X + r * ldx + k;
+        __align__(16) T v[E];
+#pragma unroll
+        for (int q = 0; q < E; q++)
+            v[q] = k + q < K ? __ldg(p + q) : T(0.f);
+        *reinterpret_cast<uint4 *>(P + i * E) = *reinterpret_cast<const uint4 *>(v);
+    }
 }
 
 }  // namespace dev
