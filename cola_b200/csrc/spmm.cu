@@ -20,6 +20,7 @@
 #include "graph.h"
 #include "spmm_kernels.cuh"
 #include "spmm_rows.cuh"
+#include "spmm_fused.cuh"
 #include "batch.h"
 
 using cola::dev::GatherSeg;
@@ -134,15 +135,76 @@ static cola_status launch_fused_geo(const FusedArgs &a, int V, cudaStream_t st)
     return launch_fused_t<TR, 32, 4, 2, VEC_Y>(a, st);
 }
 
+// Streamed form: kFusedSpan consecutive chunks a warp (longer spans leave the hub
+// columns' warps running alone: pipelined schedule, R-MAT 131 K rows, 3.9 M
+// entries, K = 64 BF16, spans of 1, 2, 4, 8, 32: 0.51, 0.43, 0.39, 0.37, 0.43 ms).
+constexpr int kFusedSpan = 8;
+
+// Where it runs: BF16 X, and FP32 X up to 32 features (the fused schedule on that
+// graph, one warp a chunk against streamed: K = 64 BF16 0.75 -> 0.34 ms, K = 32
+// FP32 0.23 -> 0.20; K = 128 FP32 through the kernel-level launcher 0.84 against
+// 0.99: there the reductions bound both and the older form keeps twice the
+// warps), when the launch has half a span for every warp of a wave (the buffer
+// schedule's 4,096-chunk launches do not: K = 32 FP32 0.95 against 1.08 ms).
+static bool fused_streams(const FusedArgs &a)
+{
+    return a.vec && (a.xdt == COLA_BFLOAT16 || a.K <= 32) &&
+           a.total >= (int64_t)sm_count() * 4 * dev::kWarpsPerBlock * (kFusedSpan / 2);
+}
+
+template <typename TR, int LG, int NV, int UNROLL, int MINB>
+static cola_status launch_stream_t(const FusedArgs &a, cudaStream_t st)
+{
+    using T = typename dev::ElemOf<TR>::T;
+    constexpr int W = LG * NV * TR::E;
+    auto fn = dev::fused_stream_kernel<TR, LG, NV, UNROLL, MINB>;
+    const int span = kFusedSpan;
+    const int64_t gx = (a.total + (int64_t)span * dev::kWarpsPerBlock - 1) / ((int64_t)span * dev::kWarpsPerBlock);
+    t_launches++;
+    fn<<<dim3((unsigned)gx, (unsigned)((a.K + W - 1) / W)), dev::kThreads, 0, st>>>(
+        a.parts, a.single, a.nparts, a.total, span, static_cast<const T *>(a.X), a.ldx, a.Y, a.ldy, a.K);
+    COLA_CUDA(cudaGetLastError());
+    return COLA_SUCCESS;
+}
+
+template <typename TR>
+static cola_status launch_stream_narrow(const FusedArgs &a, int V, cudaStream_t st)  // V <= 8 vectors a row
+{
+    if (V <= 1)
+        return launch_stream_t<TR, 1, 1, 1, 4>(a, st);
+    if (V <= 2)
+        return launch_stream_t<TR, 2, 1, 2, 4>(a, st);
+    if (V <= 4)
+        return launch_stream_t<TR, 4, 1, 4, 4>(a, st);
+    return launch_stream_t<TR, 8, 1, 4, 4>(a, st);
+}
+
+template <typename TR>
+static cola_status launch_stream_geo(const FusedArgs &a, int V, cudaStream_t st)
+{
+    if (V <= 8)
+        return launch_stream_narrow<TR>(a, V, st);
+    if (V <= 16)
+        return launch_stream_t<TR, 16, 1, 4, 4>(a, st);
+    if (V <= 32)
+        return launch_stream_t<TR, 32, 1, 4, 4>(a, st);
+    return launch_stream_t<TR, 32, 2, 4, 3>(a, st);
+}
+
 static cola_status launch_fused(const FusedArgs &a, cudaStream_t st)
 {
     if (a.total <= 0 || a.K <= 0)
         return COLA_SUCCESS;
+    const bool stream = fused_streams(a);
     if (a.xdt == COLA_FLOAT32) {
+        if (stream)
+            return launch_stream_narrow<dev::VecTraits<float>>(a, a.K / 4, st);
         if (a.vec)
             return launch_fused_geo<dev::VecTraits<float>, true>(a, a.K / 4, st);
         return launch_fused_geo<dev::ScalarTraits<float>, false>(a, a.K, st);
     }
+    if (stream)
+        return launch_stream_geo<dev::VecTraits<__nv_bfloat16>>(a, a.K / 8, st);
     if (a.vec)
         return launch_fused_geo<dev::VecTraits<__nv_bfloat16>, true>(a, a.K / 8, st);
     return launch_fused_geo<dev::ScalarTraits<__nv_bfloat16>, false>(a, a.K, st);
@@ -153,7 +215,7 @@ static bool vec_ok(cola_dtype xdt, const void *X, int64_t ldx, const void *stage
                    int64_t ldy, int K)
 {
     const int E = xdt == COLA_FLOAT32 ? 4 : 8;
-    if (K % E || ldx % E || !aligned16(X))
+    if (K % E || ldx % E || ldx > INT32_MAX / (16 / E) || !aligned16(X))
         return false;
     if (stage && (ld_stage % E || !aligned16(stage)))
         return false;

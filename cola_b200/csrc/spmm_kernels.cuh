@@ -177,6 +177,18 @@ struct ElemOf<NarrowTraits<U, B>> {
     using T = U;
 };
 
+// The vectors a remote chunk's dense row is read in: 4 features a lane, so that
+// neighbouring lanes' 16-byte reductions into FP32 Y make whole sectors (with 8
+// BF16 features a lane each of its two reductions would be half of them).
+template <typename TR>
+struct ScatterOf {
+    using type = TR;
+};
+template <>
+struct ScatterOf<VecTraits<__nv_bfloat16>> {
+    using type = NarrowTraits<__nv_bfloat16, 8>;
+};
+
 // Y[p..p+E) += a[0..E): 16-byte vector reductions when E is a multiple of 4.
 template <int E, bool VEC_Y>
 __device__ __forceinline__ void red_add(float *p, const float (&a)[E])
@@ -185,6 +197,8 @@ __device__ __forceinline__ void red_add(float *p, const float (&a)[E])
 #pragma unroll
         for (int q = 0; q < E / 4; q++)
             atomicAdd(reinterpret_cast<float4 *>(p + 4 * q), make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]));
+    } else if constexpr (VEC_Y && E == 2) {
+        atomicAdd(reinterpret_cast<float2 *>(p), make_float2(a[0], a[1]));
     } else {
 #pragma unroll
         for (int q = 0; q < E; q++)
@@ -316,11 +330,14 @@ __global__ void __launch_bounds__(kThreads, MINB) fused_spmm_kernel(const PartDe
             }
             src += k0;
             // stage the dense row on chip (registers)
-            float xs[NV][E];
+            using TS = typename ScatterOf<TR>::type;
+            constexpr int ES = TS::E, NS = NV * E / ES;
+            const int ks = gl * ES;
+            float xs[NS][ES];
 #pragma unroll
-            for (int j = 0; j < NV; j++) {
-                raw_t r = kok[j] ? TR::load(src + (gl + j * LG) * E) : TR::zero();
-                TR::unpack(r, xs[j]);
+            for (int j = 0; j < NS; j++) {
+                const typename TS::raw_t r = k0 + ks + j * LG * ES < K ? TS::load(src + ks + j * LG * ES) : TS::zero();
+                TS::unpack(r, xs[j]);
             }
             for (int base = lb; base < hb; base += 32) {
                 const int n = min(32, hb - base);
@@ -335,15 +352,15 @@ __global__ void __launch_bounds__(kThreads, MINB) fused_spmm_kernel(const PartDe
                     const int r = __shfl_sync(kFull, mr, k & 31);
                     const float v = __shfl_sync(kFull, mv, k & 31);
                     if (k < n) {
-                        float *yp = Y + (d.y_row0 + r) * ldy + k0;
+                        float *yp = Y + (d.y_row0 + r) * ldy + k0 + ks;
 #pragma unroll
-                        for (int j = 0; j < NV; j++)
-                            if (kok[j]) {
-                                float a[E];
+                        for (int j = 0; j < NS; j++)
+                            if (k0 + ks + j * LG * ES < K) {
+                                float a[ES];
 #pragma unroll
-                                for (int e = 0; e < E; e++)
+                                for (int e = 0; e < ES; e++)
                                     a[e] = v * xs[j][e];
-                                red_add<E, VEC_Y>(yp + (gl + j * LG) * E, a);
+                                red_add<ES, VEC_Y>(yp + j * LG * ES, a);
                             }
                     }
                 }

@@ -333,8 +333,9 @@ __device__ __forceinline__ int lane_id()
 // flight at 3 blocks (1.10 ms), 2 at 5 or 6 (1.35), the next row's load issued
 // as each row is added (1.64).
 // VEC_Y: rows of Y are written in vectors; else (their start is not aligned or K
-// ends inside a vector of X) element by element, X still read in vectors.
-template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC_Y = true>
+// ends inside a vector of X) element by element, X still read in vectors.  RED:
+// sums are added to Y with reductions (other warps add to the same rows).
+template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC_Y = true, bool RED = false>
 struct RowStream {
     using T = typename ElemOf<TR>::T;
     using raw_t = typename TR::raw_t;
@@ -386,7 +387,9 @@ struct RowStream {
     template <typename TO, int N>
     __device__ __forceinline__ void put(TO *p, const float (&a)[N], bool add, int left) const
     {
-        if constexpr (VEC_Y)
+        if constexpr (RED)
+            red_add<N, true>(p, a);
+        else if constexpr (VEC_Y)
             store_out<TO, N, (N > 1)>(p, a, add);
         else if (to_ws)
             store_out<TO, N, (N > 1)>(p, a, false);
@@ -497,12 +500,11 @@ struct RowStream {
     }
 
     // One batch of n entries (1..32); ends: bit i set where entry i is its
-    // row's last.
-    __device__ __forceinline__ void batch(const EntryBatch &eb, const int n, const uint32_t ends)
+    // row's last; rows: the rows that end, in order.
+    __device__ __forceinline__ void batch(const EntryBatch &eb, const int32_t *rows, const int n, const uint32_t ends)
     {
-        int done = 0;
         auto flush = [&]() {
-            const int row = eb.row[done++];
+            const int row = *rows++;
             write_row(Y + (int64_t)row * ldy + koff, accumulate);
         };
 #pragma unroll 1
@@ -601,7 +603,7 @@ __device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const i
         kpos += __popc(ends);
         if (left > 0)
             fetch();
-        rs.batch(eb, n, ends);
+        rs.batch(eb, eb.row, n, ends);
     }
     if (seg)
         rs.write_row(ba.ws + (int64_t)it * ba.ld_ws + rs.koff, false);
