@@ -16,7 +16,7 @@
 // index (csr_colIdx_l / csc_rowIdx_r), a change of primary opens a row
 // (column), the primaries at those points are csr_rowIdx_l / csc_colIdx_r and
 // their positions are the row (column) pointers.  All of it is integer work
-// bound by HBM: the sort moves 12 bytes per entry per 8-bit digit.
+// bound by HBM: the sort moves 12 bytes per entry per 8-bit digit (key and value).
 #include <algorithm>
 #include <array>
 #include <climits>
@@ -48,6 +48,22 @@ constexpr int kScanTile = kThreads * kScanItems;
 static_assert(kBins == kThreads, "one radix bin per thread");
 
 __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << (threadIdx.x & 31)) - 1u; }
+
+// The lanes whose digit is this lane's (d < kBins, or kBins: none), from one
+// ballot per digit bit: match_any takes about 50 cycles of an SM per warp, and
+// bound both radix kernels.
+__device__ __forceinline__ uint32_t same_digit(uint32_t d)
+{
+    const bool ok = d < (1u << 8);
+    uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t with = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? with : ~with;
+    }
+    return ok ? peers : 0u;
+}
 
 // ---------------------------------------------------------------------------
 // exclusive scan of n uint32 values given by a functor (three launches)
@@ -97,22 +113,25 @@ __global__ void __launch_bounds__(kThreads) scan_reduce_kernel(F f, int64_t n, u
 // One block: partial[] becomes its exclusive scan; *total = the sum.
 __global__ void __launch_bounds__(kThreads) scan_partials_kernel(uint32_t *partial, int64_t nb, uint32_t *total)
 {
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0)
-        carry = 0;
-    __syncthreads();
-    for (int64_t b0 = 0; b0 < nb; b0 += kThreads) {
-        const int64_t b = b0 + threadIdx.x;
-        const uint32_t v = b < nb ? partial[b] : 0u;
+    uint32_t carry = 0;
+    for (int64_t b0 = 0; b0 < nb; b0 += kScanTile) {
+        const int64_t b = b0 + (int64_t)threadIdx.x * kScanItems;
+        uint32_t v[kScanItems], sum = 0;
+#pragma unroll
+        for (int j = 0; j < kScanItems; j++) {
+            v[j] = b + j < nb ? partial[b + j] : 0u;
+            sum += v[j];
+        }
         uint32_t excl;
-        const uint32_t t = block_exclusive_scan(v, excl);
-        const uint32_t c = carry;
-        if (b < nb)
-            partial[b] = c + excl;
-        __syncthreads();
-        if (threadIdx.x == 0)
-            carry = c + t;
-        __syncthreads();
+        const uint32_t t = block_exclusive_scan(sum, excl);
+        uint32_t run = carry + excl;
+#pragma unroll
+        for (int j = 0; j < kScanItems; j++) {
+            if (b + j < nb)
+                partial[b + j] = run;
+            run += v[j];
+        }
+        carry += t;
     }
     if (threadIdx.x == 0)
         *total = carry;
@@ -149,6 +168,18 @@ struct KeyStartF {
     int shift;
     __device__ uint32_t operator()(int64_t i) const { return i == 0 || (k[i] >> shift) != (k[i - 1] >> shift); }
 };
+// *count += the keys that differ from the one before them.
+__global__ void count_starts_kernel(const uint64_t *__restrict__ k, int64_t n, unsigned int *count)
+{
+    unsigned int c = 0;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        c += i == 0 || k[i] != k[i - 1];
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c)
+        atomicAdd(count, c);
+}
+
 // nnz_split chunks of row i: ceil(len / gran)
 struct ChunksF {
     const int32_t *ptr;
@@ -164,28 +195,30 @@ struct ChunksF {
 // partitioning kernels
 // ---------------------------------------------------------------------------
 
-__global__ void check_coo_kernel(const int32_t *row, const int32_t *col, int64_t n, int32_t NR, int32_t NC,
+// An entry outside NR x NC is noted and sorted as (0, 0); the caller fails.
+__device__ __forceinline__ bool entry_ok(int32_t r, int32_t c, int32_t NR, int32_t NC, int64_t i,
+                                         unsigned long long *first_bad)
+{
+    if (r >= 0 && r < NR && c >= 0 && c < NC)
+        return true;
+    atomicMin(first_bad, (unsigned long long)i);
+    return false;
+}
+
+__global__ void make_keys_kernel(const int32_t *row, const int32_t *col, const float *val, int64_t n, int32_t N,
+                                 uint32_t npp, int sb, int gshift, uint64_t *key, float *v,
                                  unsigned long long *first_bad)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t r = row[i], c = col[i];
-        if (r < 0 || r >= NR || c < 0 || c >= NC)
-            atomicMin(first_bad, (unsigned long long)i);
-    }
-}
-
-__global__ void make_keys_kernel(const int32_t *row, const int32_t *col, int64_t n, uint32_t npp, int sb, int gshift,
-                                 uint64_t *key, uint32_t *idx)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = (uint32_t)row[i], c = (uint32_t)col[i];
+        const bool ok = entry_ok(row[i], col[i], N, N, i, first_bad);
+        const uint32_t r = ok ? (uint32_t)row[i] : 0u, c = ok ? (uint32_t)col[i] : 0u;
         const uint32_t p = r / npp, lb = p * npp;
         const bool local = c / npp == p;
         const uint64_t g = 2ull * p + (local ? 0u : 1u);
         const uint64_t prim = local ? r - lb : c;
         const uint64_t sec = local ? c - lb : r - lb;
         key[i] = g << gshift | prim << sb | sec;
-        idx[i] = (uint32_t)i;
+        v[i] = val ? val[i] : 1.0f;
     }
 }
 
@@ -196,80 +229,125 @@ __global__ void __launch_bounds__(kThreads) radix_hist_kernel(const uint64_t *ke
 {
     __shared__ uint32_t h[kBins];
     h[threadIdx.x] = 0;
-    __syncthreads();
     const int64_t tile0 = (int64_t)blockIdx.x * kTile;
-    for (int r = 0; r < kItems; r++) {
+    uint32_t d[kItems];
+#pragma unroll
+    for (int r = 0; r < kItems; r++) {  // every load before the first count
         const int64_t i = tile0 + r * kThreads + threadIdx.x;
-        const uint32_t d = i < n ? (uint32_t)(key[i] >> shift) & (kBins - 1) : (uint32_t)kBins;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        if (d < kBins && (peers & lanemask_lt()) == 0)
-            atomicAdd(&h[d], (uint32_t)__popc(peers));
+        d[r] = i < n ? (uint32_t)(key[i] >> shift) & (kBins - 1) : (uint32_t)kBins;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; r++) {
+        const uint32_t peers = same_digit(d[r]);
+        if (d[r] < kBins && (peers & lanemask_lt()) == 0)
+            atomicAdd(&h[d[r]], (uint32_t)__popc(peers));
     }
     __syncthreads();
     hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// Stable scatter of one tile: entries keep their order within each digit.
-// Rounds of kThreads consecutive entries; inside a round a warp ranks its
-// lanes per digit (match_any), warps are ranked per digit in shared memory,
-// and rounds follow one another per digit through base[].
-__global__ void __launch_bounds__(kThreads) radix_scatter_kernel(const uint64_t *kin, const uint32_t *vin,
-                                                                 uint64_t *kout, uint32_t *vout, int64_t n, int shift,
+// Stable scatter of one tile: entries keep their order within each digit.  A
+// warp owns kItems * 32 consecutive entries and ranks its lanes per digit 32 at a
+// time against its own counters; the block then orders the
+// tile by digit in shared memory, so that each digit's entries are written as
+// one run.  Bound by HBM (24 bytes per entry).  Writing every entry straight to
+// its place, with two block-wide waits per 256 entries, took 0.28 ms per digit
+// of a 14 M-entry sort, the counts 0.095; now 0.14 and 0.06.
+__global__ void __launch_bounds__(kThreads) radix_scatter_kernel(const uint64_t *kin, const float *vin,
+                                                                 uint64_t *kout, float *vout, int64_t n, int shift,
                                                                  int64_t ntiles, const uint32_t *hist_scan)
 {
-    __shared__ uint32_t base[kBins];
-    __shared__ uint32_t wcnt[kWarps][kBins];
-    __shared__ uint32_t wpos[kWarps][kBins];
-    const int t = threadIdx.x, w = t >> 5;
-    base[t] = hist_scan[(int64_t)t * ntiles + blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < kWarps; k++)
-        wcnt[k][t] = 0;
-    __syncthreads();
+    __shared__ uint64_t sk[kTile];            // the tile by digit: keys, then values
+    __shared__ uint32_t wcnt[kWarps][kBins];  // a warp's entries per digit, then those of the warps before it
+    __shared__ uint32_t lstart[kBins];        // first place of a digit in the tile
+    __shared__ uint32_t gbase[kBins];         // its global place, minus that
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
     const int64_t tile0 = (int64_t)blockIdx.x * kTile;
-    for (int r = 0; r < kItems; r++) {
-        if (tile0 + (int64_t)r * kThreads >= n)
-            break;  // uniform across the block
-        const int64_t i = tile0 + r * kThreads + t;
-        const bool valid = i < n;
-        const uint64_t k = valid ? kin[i] : 0ull;
-        const uint32_t v = valid ? vin[i] : 0u;
-        const uint32_t d = valid ? (uint32_t)(k >> shift) & (kBins - 1) : (uint32_t)kBins;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        const uint32_t rank = __popc(peers & lanemask_lt());
-        if (valid && rank == 0)
-            wcnt[w][d] = __popc(peers);
-        __syncthreads();
-        uint32_t run = base[t];
+    const int cnt = (int)min((int64_t)kTile, n - tile0);
+    uint64_t k[kItems];
+    float v[kItems];
+    uint32_t rk[kItems];
+    const int at0 = w * (kItems * 32) + lane;
 #pragma unroll
-        for (int q = 0; q < kWarps; q++) {
-            const uint32_t c = wcnt[q][t];
-            wpos[q][t] = run;
-            run += c;
-            wcnt[q][t] = 0;
+    for (int r = 0; r < kItems; r++)
+        if (at0 + r * 32 < cnt) {
+            k[r] = kin[tile0 + at0 + r * 32];
+            v[r] = vin[tile0 + at0 + r * 32];
         }
-        base[t] = run;
-        __syncthreads();
-        if (valid) {
-            const uint32_t pos = wpos[w][d] + rank;
-            kout[pos] = k;
-            vout[pos] = v;
+    for (int b = lane; b < kBins; b += 32)
+        wcnt[w][b] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kItems; r++) {
+        const bool ok = at0 + r * 32 < cnt;
+        const uint32_t d = ok ? (uint32_t)(k[r] >> shift) & (kBins - 1) : (uint32_t)kBins;
+        const uint32_t peers = same_digit(d);
+        const int first = ok ? __ffs(peers) - 1 : lane;
+        uint32_t before = 0;
+        if (ok && lane == first) {
+            before = wcnt[w][d];
+            wcnt[w][d] = before + __popc(peers);
+        }
+        rk[r] = __shfl_sync(0xffffffffu, before, first) + __popc(peers & lanemask_lt());
+        __syncwarp();
+    }
+    __syncthreads();
+    uint32_t run = 0;  // thread t: digit t
+#pragma unroll
+    for (int q = 0; q < kWarps; q++) {
+        const uint32_t c = wcnt[q][t];
+        wcnt[q][t] = run;
+        run += c;
+    }
+    uint32_t excl;
+    block_exclusive_scan(run, excl);
+    lstart[t] = excl;
+    gbase[t] = hist_scan[(int64_t)t * ntiles + blockIdx.x] - excl;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; r++)
+        if (at0 + r * 32 < cnt) {
+            const uint32_t d = (uint32_t)(k[r] >> shift) & (kBins - 1);
+            rk[r] += lstart[d] + wcnt[w][d];
+            sk[rk[r]] = k[r];
+        }
+    __syncthreads();
+    uint32_t pos[kItems];
+#pragma unroll
+    for (int r = 0; r < kItems; r++) {
+        const int i = t + r * kThreads;
+        if (i < cnt) {
+            const uint64_t key = sk[i];
+            pos[r] = gbase[(uint32_t)(key >> shift) & (kBins - 1)] + (uint32_t)i;
+            kout[pos[r]] = key;
         }
     }
+    __syncthreads();
+    float *sv = reinterpret_cast<float *>(sk);
+#pragma unroll
+    for (int r = 0; r < kItems; r++)
+        if (at0 + r * 32 < cnt)
+            sv[rk[r]] = v[r];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; r++)
+        if (t + r * kThreads < cnt)
+            vout[pos[r]] = sv[t + r * kThreads];
 }
 
 // One thread per run of equal keys: the unique key and its values summed in
-// input order (1.0 each without values).
-__global__ void dedupe_kernel(const uint64_t *key, const uint32_t *idx, const float *val, int64_t n,
-                              const uint32_t *upos, uint64_t *ukey, float *uval)
+// input order.
+__global__ void dedupe_kernel(const uint64_t *key, const float *val, int64_t n, const uint32_t *upos, uint64_t *ukey,
+                              float *uval)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t k = key[i];
         if (i > 0 && key[i - 1] == k)
             continue;
-        float v = val ? val[idx[i]] : 1.0f;
+        float v = val[i];
         for (int64_t j = i + 1; j < n && key[j] == k; j++)
-            v += val ? val[idx[j]] : 1.0f;
+            v += val[j];
         const uint32_t u = upos[i];
         ukey[u] = k;
         uval[u] = v;
@@ -394,12 +472,15 @@ __global__ void relabel_kernel(const int32_t *row, const int32_t *col, int64_t n
 // host upload derives from the partitions (spmm.cu graph_upload)
 // ---------------------------------------------------------------------------
 
-__global__ void make_row_keys_kernel(const int32_t *row, const int32_t *col, int64_t n, int cb, uint64_t *key,
-                                     uint32_t *idx)
+__global__ void make_row_keys_kernel(const int32_t *__restrict__ row, const int32_t *__restrict__ col,
+                                     const float *__restrict__ val, int64_t n, int32_t NR, int32_t NC, int cb,
+                                     uint64_t *__restrict__ key, float *__restrict__ v, unsigned long long *first_bad)
 {
+#pragma unroll 4
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        key[i] = (uint64_t)(uint32_t)row[i] << cb | (uint32_t)col[i];
-        idx[i] = (uint32_t)i;
+        const bool ok = entry_ok(row[i], col[i], NR, NC, i, first_bad);
+        key[i] = ok ? (uint64_t)(uint32_t)row[i] << cb | (uint32_t)col[i] : 0ull;
+        v[i] = val ? val[i] : 1.0f;
     }
 }
 
@@ -420,10 +501,25 @@ __global__ void row_ptr_kernel(const uint64_t *ukey, int64_t U, int cb, int64_t 
     }
 }
 
-__global__ void row_cols_kernel(const uint64_t *ukey, int64_t U, uint64_t cmask, int32_t *rv_col)
+// The row view's columns and values, and the number of entries whose column lies
+// in the row's own partition (the local block).
+__global__ void row_entries_kernel(const uint64_t *__restrict__ ukey, const float *__restrict__ uval, int64_t U,
+                                   int cb, uint32_t npp, int32_t *__restrict__ rv_col, float *__restrict__ rv_val,
+                                   unsigned long long *local)
 {
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < U; u += (int64_t)gridDim.x * blockDim.x)
-        rv_col[u] = (int32_t)(ukey[u] & cmask);
+    const uint64_t cmask = (1ull << cb) - 1;
+    uint32_t c = 0;
+#pragma unroll 4
+    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < U; u += (int64_t)gridDim.x * blockDim.x) {
+        const uint64_t k = ukey[u];
+        const uint32_t r = (uint32_t)(k >> cb), x = (uint32_t)(k & cmask);
+        rv_col[u] = (int32_t)x;
+        rv_val[u] = uval[u];
+        c += r / npp == x / npp;
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c)
+        atomicAdd(local, (unsigned long long)c);
 }
 
 // 1 per hub row (more than thr entries)
@@ -628,21 +724,6 @@ __global__ void task_write_kernel(const int64_t *ptr, const int32_t *next, int64
     }
 }
 
-// entries whose column lies in the row's own partition (the local block)
-__global__ void count_local_kernel(const uint64_t *ukey, int64_t U, int cb, uint32_t npp,
-                                   unsigned long long *local)
-{
-    unsigned long long c = 0;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < U; u += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = (uint32_t)(ukey[u] >> cb), k = (uint32_t)(ukey[u] & ((1ull << cb) - 1));
-        c += r / npp == k / npp;
-    }
-    for (int o = 16; o > 0; o >>= 1)
-        c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c)
-        atomicAdd(local, c);
-}
-
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -820,46 +901,79 @@ static cola_status exclusive_scan(F f, int64_t n, uint32_t *out, uint32_t *d_tot
     return COLA_SUCCESS;
 }
 
-// Every entry inside NR rows x NC columns (NC < 0: NC = NR).
-static cola_status check_range(const int32_t *row, const int32_t *col, int64_t n, int32_t N, Scratch &sc,
-                               const char *who, int32_t NC = -1)
+// The first entry outside N x NC that the key kernel noted.
+static cola_status fail_range(unsigned long long bad, const int32_t *row, const int32_t *col, int32_t N, int32_t NC,
+                              const char *who)
 {
-    if (NC < 0)
-        NC = N;
-    unsigned long long *bad = nullptr, h_bad = 0;
-    COLA_TRY(sc.get(bad, 1));
-    COLA_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(*bad), sc.st));
-    check_coo_kernel<<<grid_stride_blocks(n), 256, 0, sc.st>>>(row, col, n, N, NC, bad);
-    t_launches++;
-    COLA_CUDA(cudaGetLastError());
-    COLA_CUDA(cudaMemcpyAsync(&h_bad, bad, sizeof(h_bad), cudaMemcpyDeviceToHost, sc.st));
-    COLA_CUDA(cudaStreamSynchronize(sc.st));
-    if (h_bad != ULLONG_MAX) {
-        int32_t r = 0, c = 0;
-        cudaMemcpy(&r, row + h_bad, 4, cudaMemcpyDeviceToHost);
-        cudaMemcpy(&c, col + h_bad, 4, cudaMemcpyDeviceToHost);
-        return fail(COLA_ERROR_INVALID_ARGUMENT, "%s: entry %llu (%d, %d) outside %d x %d", who, h_bad, r, c, N, NC);
-    }
-    return COLA_SUCCESS;
+    int32_t r = 0, c = 0;
+    cudaMemcpy(&r, row + bad, 4, cudaMemcpyDeviceToHost);
+    cudaMemcpy(&c, col + bad, 4, cudaMemcpyDeviceToHost);
+    return fail(COLA_ERROR_INVALID_ARGUMENT, "%s: entry %llu (%d, %d) outside %d x %d", who, bad, r, c, N, NC);
 }
 
-// Stable LSD radix sort of (key, id) pairs by the low key_bits bits of the
-// keys: on return k0/v0 point at the sorted pairs, k1/v1 at the other buffers.
-static cola_status radix_sort_pairs(uint64_t *&k0, uint32_t *&v0, uint64_t *&k1, uint32_t *&v1, int64_t n,
-                                    int key_bits, uint32_t *hist, uint32_t *d_total, Scratch &sc)
+// Buffers of one sort of n (key, value) pairs and what is left of them.
+struct SortBuf {
+    uint64_t *k0 = nullptr, *k1 = nullptr;
+    float *v0 = nullptr, *v1 = nullptr;
+    uint32_t *hist = nullptr, *d_total = nullptr;
+    unsigned long long *bad = nullptr;
+    static size_t bytes(int64_t n)
+    {
+        const int64_t ntiles = (n + kTile - 1) / kTile;
+        return 2 * (12 * (size_t)n + 512) + 4 * (size_t)ntiles * kBins + 1024 +
+               (size_t)(kMaxPasses + 1) * (4 * (size_t)((ntiles * kBins + kScanTile - 1) / kScanTile) + 512);
+    }
+    static constexpr int kMaxPasses = 64 / kDigitBits;
+    cola_status get(int64_t n, Scratch &sc)
+    {
+        COLA_TRY(sc.get(k0, n));
+        COLA_TRY(sc.get(k1, n));
+        COLA_TRY(sc.get(v0, n));
+        COLA_TRY(sc.get(v1, n));
+        COLA_TRY(sc.get(hist, (n + kTile - 1) / kTile * kBins));
+        COLA_TRY(sc.get(d_total, 1));
+        COLA_TRY(sc.get(bad, 1));
+        COLA_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(*bad), sc.st));
+        return COLA_SUCCESS;
+    }
+};
+
+// Sorts the pairs in k0 / v0 by the low key_bits bits of the keys (stable LSD
+// radix sort) and merges equal keys (values summed in input order): on return
+// k0 / v0 hold the U unique pairs and k1 / v1 are free.  bad: the noted entry,
+// or ULLONG_MAX.
+static cola_status sort_unique(SortBuf &b, int64_t n, int key_bits, uint32_t &U, unsigned long long &bad, Scratch &sc)
 {
     const int64_t ntiles = (n + kTile - 1) / kTile;
     for (int shift = 0; shift < key_bits; shift += kDigitBits) {
-        radix_hist_kernel<<<(unsigned)ntiles, kThreads, 0, sc.st>>>(k0, n, shift, ntiles, hist);
+        radix_hist_kernel<<<(unsigned)ntiles, kThreads, 0, sc.st>>>(b.k0, n, shift, ntiles, b.hist);
         t_launches++;
         COLA_CUDA(cudaGetLastError());
-        COLA_TRY(exclusive_scan(ArrayF{hist}, ntiles * kBins, hist, d_total, nullptr, sc));
-        radix_scatter_kernel<<<(unsigned)ntiles, kThreads, 0, sc.st>>>(k0, v0, k1, v1, n, shift, ntiles, hist);
+        COLA_TRY(exclusive_scan(ArrayF{b.hist}, ntiles * kBins, b.hist, b.d_total, nullptr, sc));
+        radix_scatter_kernel<<<(unsigned)ntiles, kThreads, 0, sc.st>>>(b.k0, b.v0, b.k1, b.v1, n, shift, ntiles,
+                                                                       b.hist);
         t_launches++;
         COLA_CUDA(cudaGetLastError());
-        std::swap(k0, k1);
-        std::swap(v0, v1);
+        std::swap(b.k0, b.k1);
+        std::swap(b.v0, b.v1);
     }
+    COLA_CUDA(cudaMemsetAsync(b.d_total, 0, sizeof(uint32_t), sc.st));
+    count_starts_kernel<<<grid_stride_blocks(n), 256, 0, sc.st>>>(b.k0, n, b.d_total);
+    t_launches++;
+    COLA_CUDA(cudaGetLastError());
+    COLA_CUDA(cudaMemcpyAsync(&U, b.d_total, sizeof U, cudaMemcpyDeviceToHost, sc.st));
+    COLA_CUDA(cudaMemcpyAsync(&bad, b.bad, sizeof bad, cudaMemcpyDeviceToHost, sc.st));
+    COLA_CUDA(cudaStreamSynchronize(sc.st));
+    if ((int64_t)U == n || bad != ULLONG_MAX)
+        return COLA_SUCCESS;  // nothing to merge
+    uint32_t *upos = nullptr;
+    COLA_TRY(sc.get(upos, n));
+    COLA_TRY(exclusive_scan(KeyStartF{b.k0, 0}, n, upos, b.d_total, nullptr, sc));
+    dedupe_kernel<<<grid_stride_blocks(n), 256, 0, sc.st>>>(b.k0, b.v0, n, upos, b.k1, b.v1);
+    t_launches++;
+    COLA_CUDA(cudaGetLastError());
+    std::swap(b.k0, b.k1);
+    std::swap(b.v0, b.v1);
     return COLA_SUCCESS;
 }
 
@@ -899,45 +1013,29 @@ static cola_status partition_build_device(int32_t N, int64_t nnz, const int32_t 
         return COLA_SUCCESS;
     }
     Scratch sc(st);
-    const int64_t ntiles = (nnz + kTile - 1) / kTile;
     {
-        // every buffer below, each rounded to 256 bytes, plus the scans' block sums
+        // the sort's buffers, the output arrays, the scans' block sums
         const size_t n = (size_t)nnz, a = 256;
-        const size_t scan_blocks = (size_t)((std::max<int64_t>(ntiles * kBins, nnz) + kScanTile - 1) / kScanTile) + 1;
-        const size_t bytes = 2 * (8 * n + a) + 2 * (4 * n + a) + (4 * (size_t)ntiles * kBins + a) + 4 * (4 * n + a) +
-                             (4 * (n + (size_t)G) + a) + 2 * (8 * ((size_t)G + 1) + a) + 2 * a +
-                             (2 * 6 + 16) * (4 * scan_blocks + a);
+        const size_t scan_blocks = (n + kScanTile - 1) / kScanTile + 1;
+        const size_t bytes = SortBuf::bytes(nnz) + 2 * (4 * n + a) + (4 * (n + (size_t)G) + a) +
+                             2 * (8 * ((size_t)G + 1) + a) + 2 * a + 4 * (4 * scan_blocks + a);
         COLA_TRY(sc.reserve(bytes));
     }
-    COLA_TRY(check_range(row, col, nnz, N, sc, who));
-
-    // sort
-    uint64_t *k0 = nullptr, *k1 = nullptr;
-    uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr, *d_total = nullptr;
-    COLA_TRY(sc.get(k0, nnz));
-    COLA_TRY(sc.get(k1, nnz));
-    COLA_TRY(sc.get(v0, nnz));
-    COLA_TRY(sc.get(v1, nnz));
-    COLA_TRY(sc.get(hist, ntiles * kBins));
-    COLA_TRY(sc.get(d_total, 1));
-    make_keys_kernel<<<grid_stride_blocks(nnz), 256, 0, st>>>(row, col, nnz, (uint32_t)(npp > 0 ? npp : 1), sb,
-                                                              gshift, k0, v0);
+    SortBuf sb_;
+    COLA_TRY(sb_.get(nnz, sc));
+    make_keys_kernel<<<grid_stride_blocks(nnz), 256, 0, st>>>(row, col, val, nnz, N, (uint32_t)(npp > 0 ? npp : 1), sb,
+                                                              gshift, sb_.k0, sb_.v0, sb_.bad);
     t_launches++;
     COLA_CUDA(cudaGetLastError());
-    COLA_TRY(radix_sort_pairs(k0, v0, k1, v1, nnz, key_bits, hist, d_total, sc));
-    // merge duplicates: unique keys into k1, summed values
-    uint32_t *upos = nullptr;
-    float *uval = nullptr;
-    uint32_t U = 0;
-    COLA_TRY(sc.get(upos, nnz));
-    COLA_TRY(exclusive_scan(KeyStartF{k0, 0}, nnz, upos, d_total, &U, sc));
-    COLA_TRY(sc.get(uval, U));
-    uint64_t *ukey = k1;
-    dedupe_kernel<<<grid_stride_blocks(nnz), 256, 0, st>>>(k0, v0, val, nnz, upos, ukey, uval);
-    t_launches++;
-    COLA_CUDA(cudaGetLastError());
+    uint32_t U = 0, *d_total = sb_.d_total;
+    unsigned long long bad = ULLONG_MAX;
+    COLA_TRY(sort_unique(sb_, nnz, key_bits, U, bad, sc));
+    if (bad != ULLONG_MAX)
+        return fail_range(bad, row, col, N, N, who);
+    const uint64_t *ukey = sb_.k0;
+    const float *uval = sb_.v0;
     // rows (local) / columns (remote): runs of equal primary within a group
-    uint32_t *spos = upos, *seg_start = v1;  // both free again (U <= nnz)
+    uint32_t *spos = reinterpret_cast<uint32_t *>(sb_.k1), *seg_start = spos + nnz;  // the free key buffer (U <= nnz)
     uint32_t S = 0;
     COLA_TRY(exclusive_scan(KeyStartF{ukey, sb}, U, spos, d_total, &S, sc));
     seg_start_kernel<<<grid_stride_blocks(U), 256, 0, st>>>(ukey, U, spos, sb, seg_start);
@@ -1038,64 +1136,43 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
 
     Scratch sc(st);
     {
-        const size_t n = (size_t)nnz, a = 256;
-        const int64_t ntiles = (nnz + kTile - 1) / kTile;
-        const size_t rows = (size_t)N + 1;
-        const size_t scan_blocks = (size_t)((std::max<int64_t>(std::max<int64_t>(ntiles * kBins, nnz), N + 1) +
-                                             kScanTile - 1) / kScanTile) + 1;
-        // sort keys and ids (x2), digit counts, unique positions, values and
-        // columns, row pointers, hub and segment positions, the task packing's
-        // row arrays, small values, the scans' block sums
-        const size_t bytes = 2 * (8 * n + a) + 2 * (4 * n + a) + (4 * (size_t)ntiles * kBins + a) + 3 * (4 * n + a) +
-                             (8 * rows + a) + 8 * (4 * (rows + kTaskBlock) + a) + 6 * a + 28 * (4 * scan_blocks + a);
+        // the sort's buffers, row pointers, hub, segment and row positions, the task
+        // packing's row arrays, small values, the scans' block sums
+        const size_t a = 256, rows = (size_t)N + 1, scan_blocks = rows / kScanTile + 2;
+        const size_t bytes = SortBuf::bytes(nnz) + (8 * rows + a) + 8 * (4 * (rows + kTaskBlock) + a) + 6 * a +
+                             8 * (4 * scan_blocks + a);
         COLA_TRY(sc.reserve(bytes));
     }
-    if (nnz > 0)
-        COLA_TRY(check_range(row, col, nnz, N, sc, who, NC));
-    uint32_t *d_total = nullptr;
-    COLA_TRY(sc.get(d_total, 1));
-    uint64_t *ukey = nullptr;
-    float *uval = nullptr;
+    SortBuf sb;
     uint32_t U = 0;
     if (nnz > 0) {
-        uint64_t *k0 = nullptr, *k1 = nullptr;
-        uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr, *upos = nullptr;
-        const int64_t ntiles = (nnz + kTile - 1) / kTile;
-        COLA_TRY(sc.get(k0, nnz));
-        COLA_TRY(sc.get(k1, nnz));
-        COLA_TRY(sc.get(v0, nnz));
-        COLA_TRY(sc.get(v1, nnz));
-        COLA_TRY(sc.get(hist, ntiles * kBins));
-        make_row_keys_kernel<<<grid_stride_blocks(nnz), 256, 0, st>>>(row, col, nnz, cb, k0, v0);
+        unsigned long long bad = ULLONG_MAX;
+        COLA_TRY(sb.get(nnz, sc));
+        make_row_keys_kernel<<<grid_stride_blocks(nnz), 256, 0, st>>>(row, col, val, nnz, N, NC, cb, sb.k0, sb.v0,
+                                                                      sb.bad);
         t_launches++;
         COLA_CUDA(cudaGetLastError());
-        COLA_TRY(radix_sort_pairs(k0, v0, k1, v1, nnz, 2 * cb, hist, d_total, sc));
-        COLA_TRY(sc.get(upos, nnz));
-        COLA_TRY(exclusive_scan(KeyStartF{k0, 0}, nnz, upos, d_total, &U, sc));
-        COLA_TRY(sc.get(uval, U));
-        ukey = k1;
-        dedupe_kernel<<<grid_stride_blocks(nnz), 256, 0, st>>>(k0, v0, val, nnz, upos, ukey, uval);
-        t_launches++;
-        COLA_CUDA(cudaGetLastError());
+        COLA_TRY(sort_unique(sb, nnz, 2 * cb, U, bad, sc));
+        if (bad != ULLONG_MAX)
+            return fail_range(bad, row, col, N, NC, who);
     }
-    // row pointers and columns
+    // row pointers
     int64_t *rv_ptr = nullptr;
-    int32_t *rv_col = nullptr;
     COLA_TRY(sc.get(rv_ptr, (int64_t)N + 1));
-    COLA_TRY(sc.get(rv_col, U));
     if (U > 0) {
-        row_ptr_kernel<<<grid_stride_blocks((int64_t)N + 1), 256, 0, st>>>(ukey, U, cb, N, rv_ptr);
-        row_cols_kernel<<<grid_stride_blocks(U), 256, 0, st>>>(ukey, U, cb >= 64 ? ~0ull : (1ull << cb) - 1, rv_col);
-        t_launches += 2;
+        row_ptr_kernel<<<grid_stride_blocks((int64_t)N + 1), 256, 0, st>>>(sb.k0, U, cb, N, rv_ptr);
+        t_launches++;
     } else {
         COLA_CUDA(cudaMemsetAsync(rv_ptr, 0, ((size_t)N + 1) * 8, st));
     }
     COLA_CUDA(cudaGetLastError());
     // hub rows and their segments; the tasks of the other rows
-    uint32_t nhub = 0, nseg = 0, ntask = 0, nnz_rows = 0;
+    uint32_t *d_tot = nullptr;  // hubs, segments, rows with entries, tasks
     uint32_t *hubpos = nullptr, *segoff = nullptr, *nzpos = nullptr, *tstart = nullptr, *tpos = nullptr;
     int32_t *tnext = nullptr, *texit = nullptr, *texit2 = nullptr, *tentry = nullptr, *tsuper = nullptr;
     const int64_t ntb = ((int64_t)N + kTaskBlock - 1) / kTaskBlock, nsuper = (ntb + kTaskSuper - 1) / kTaskSuper;
+    COLA_TRY(sc.get(d_tot, 4));
+    COLA_CUDA(cudaMemsetAsync(d_tot, 0, 4 * sizeof(uint32_t), st));
     COLA_TRY(sc.get(hubpos, N));
     COLA_TRY(sc.get(segoff, N));
     COLA_TRY(sc.get(nzpos, N));
@@ -1106,9 +1183,9 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     COLA_TRY(sc.get(texit2, nsuper * kTaskBlock));
     COLA_TRY(sc.get(tentry, ntb));
     COLA_TRY(sc.get(tsuper, nsuper));
-    COLA_TRY(exclusive_scan(HubF{rv_ptr, thr}, N, hubpos, d_total, &nhub, sc));
-    COLA_TRY(exclusive_scan(SegCountF{rv_ptr, thr, seg}, N, segoff, d_total, &nseg, sc));
-    COLA_TRY(exclusive_scan(SomeF{rv_ptr}, N, nzpos, d_total, &nnz_rows, sc));
+    COLA_TRY(exclusive_scan(HubF{rv_ptr, thr}, N, hubpos, d_tot, nullptr, sc));
+    COLA_TRY(exclusive_scan(SegCountF{rv_ptr, thr, seg}, N, segoff, d_tot + 1, nullptr, sc));
+    COLA_TRY(exclusive_scan(SomeF{rv_ptr}, N, nzpos, d_tot + 2, nullptr, sc));
     if (N > 0) {
         task_next_kernel<<<grid_stride_blocks(N), 256, 0, st>>>(rv_ptr, N, thr, te, hubpos, tnext);
         task_exit_kernel<<<(unsigned)ntb, kThreads, 0, st>>>(tnext, N, texit);
@@ -1119,18 +1196,12 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
         task_starts_kernel<<<(unsigned)ntb, kThreads, 0, st>>>(rv_ptr, tnext, N, thr, tentry, tstart);
         t_launches += 5;
         COLA_CUDA(cudaGetLastError());
-        COLA_TRY(exclusive_scan(ArrayF{tstart}, N, tpos, d_total, &ntask, sc));
+        COLA_TRY(exclusive_scan(ArrayF{tstart}, N, tpos, d_tot + 3, nullptr, sc));
     }
-    // nnz in the partitions' local blocks
-    unsigned long long *d_local = nullptr, h_local = 0;
-    COLA_TRY(sc.get(d_local, 1));
-    COLA_CUDA(cudaMemsetAsync(d_local, 0, sizeof(*d_local), st));
-    if (U > 0) {
-        count_local_kernel<<<grid_stride_blocks(U), 256, 0, st>>>(ukey, U, cb, (uint32_t)std::max<int64_t>(npp, 1),
-                                                                  d_local);
-        t_launches++;
-    }
-    COLA_CUDA(cudaMemcpyAsync(&h_local, d_local, sizeof(h_local), cudaMemcpyDeviceToHost, st));
+    uint32_t h_tot[4] = {0, 0, 0, 0};
+    COLA_CUDA(cudaMemcpyAsync(h_tot, d_tot, sizeof h_tot, cudaMemcpyDeviceToHost, st));
+    COLA_CUDA(cudaStreamSynchronize(st));
+    const uint32_t nhub = h_tot[0], nseg = h_tot[1], nnz_rows = h_tot[2], ntask = h_tot[3];
 
     // the graph's own arena, in the order and alignment of the host upload
     size_t total = 0;
@@ -1154,10 +1225,18 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     char *base = static_cast<char *>(g->dmem);
     COLA_CUDA(cudaMemcpyAsync(base + o_ptr, rv_ptr, ((size_t)N + 1) * 8, cudaMemcpyDeviceToDevice, st));
     COLA_CUDA(cudaMemsetAsync(base + o_q, 0, qbytes, st));
+    // columns, values, and the number of entries in the partitions' local blocks
+    unsigned long long *d_local = nullptr, h_local = 0;
+    COLA_TRY(sc.get(d_local, 1));
+    COLA_CUDA(cudaMemsetAsync(d_local, 0, sizeof(*d_local), st));
     if (U > 0) {
-        COLA_CUDA(cudaMemcpyAsync(base + o_col, rv_col, (size_t)U * 4, cudaMemcpyDeviceToDevice, st));
-        COLA_CUDA(cudaMemcpyAsync(base + o_val, uval, (size_t)U * 4, cudaMemcpyDeviceToDevice, st));
+        row_entries_kernel<<<grid_stride_blocks(U), 256, 0, st>>>(
+            sb.k0, sb.v0, U, cb, (uint32_t)std::max<int64_t>(npp, 1), reinterpret_cast<int32_t *>(base + o_col),
+            reinterpret_cast<float *>(base + o_val), d_local);
+        t_launches++;
+        COLA_CUDA(cudaGetLastError());
     }
+    COLA_CUDA(cudaMemcpyAsync(&h_local, d_local, sizeof(h_local), cudaMemcpyDeviceToHost, st));
     const int64_t *ptr_final = reinterpret_cast<const int64_t *>(base + o_ptr);
     if (N > 0) {
         dev::WorkItem *item = reinterpret_cast<dev::WorkItem *>(base + o_item);
