@@ -69,8 +69,8 @@ static void batch_release(cola_batch *b)
         cudaGraphExecDestroy(b->cexec);
     if (b->cgraph)
         cudaGraphDestroy(b->cgraph);
-    cudaFree(b->d_desc);
-    cudaFree(b->d_ws);
+    device_free(b->d_desc);
+    device_free(b->d_ws);
     if (b->own_graphs)
         for (cola_graph *g : b->graphs)
             graph_release(g);

@@ -759,10 +759,10 @@ struct Scratch {
     }
     cola_status alloc(void *&q, size_t bytes)
     {
-        const cudaError_t e = cudaMallocAsync(&q, bytes, st);
+        const cudaError_t e = scratch_alloc(&q, bytes, st);
         if (e != cudaSuccess)
             return fail(e == cudaErrorMemoryAllocation ? COLA_ERROR_OUT_OF_MEMORY : COLA_ERROR_CUDA,
-                        "device preprocessing: cudaMallocAsync(%zu): %s", bytes, cudaGetErrorString(e));
+                        "device preprocessing: %zu bytes: %s", bytes, cudaGetErrorString(e));
         ptrs.push_back(q);
         return COLA_SUCCESS;
     }
@@ -1220,7 +1220,7 @@ static cola_status graph_build_device(int32_t N, int64_t nnz, const int32_t *row
     const size_t o_nz = place(((size_t)nnz_rows + dev::kRowPad) * 4), o_empty = place((size_t)nempty * 4);
     const size_t qbytes = (dev::kMaxItemQueues + 1) * sizeof(unsigned int), o_q = place(qbytes);
     total = std::max<size_t>(total, 256);
-    COLA_CUDA(cudaMalloc(&g->dmem, total));
+    COLA_CUDA(device_alloc(&g->dmem, total));
     g->dbytes = total;
     char *base = static_cast<char *>(g->dmem);
     COLA_CUDA(cudaMemcpyAsync(base + o_ptr, rv_ptr, ((size_t)N + 1) * 8, cudaMemcpyDeviceToDevice, st));

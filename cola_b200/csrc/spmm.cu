@@ -853,11 +853,10 @@ cola_status ensure(void *&p, size_t &have, size_t need)
 {
     if (have >= need)
         return COLA_SUCCESS;
-    if (p)
-        COLA_CUDA(cudaFree(p));
+    device_free(p);
     p = nullptr;
     have = 0;
-    COLA_CUDA(cudaMalloc(&p, need));
+    COLA_CUDA(device_alloc(&p, need));
     have = need;
     return COLA_SUCCESS;
 }
@@ -884,12 +883,12 @@ void graph_release(cola_graph *g)
     int cur = 0;
     cudaGetDevice(&cur);
     cudaSetDevice(g->device);
-    cudaFree(g->dmem);
-    cudaFree(g->ppl_buf);
-    cudaFree(g->stage_buf);
-    cudaFree(g->ws);
-    cudaFree(g->ws_hub);
-    cudaFree(g->x_pad);
+    device_free(g->dmem);
+    device_free(g->ppl_buf);
+    device_free(g->stage_buf);
+    device_free(g->ws);
+    device_free(g->ws_hub);
+    device_free(g->x_pad);
     host_pipe_release(g->host_pipe);
     cudaSetDevice(cur);
     delete g;
@@ -1060,7 +1059,7 @@ cola_status graph_upload(const cola_partition_set *ps, const cola_upload_opts *o
         o_queue = ar.add(nullptr, (dev::kMaxItemQueues + 1) * sizeof(unsigned int));  // zero in the image
     }
     ar.total = std::max<size_t>(ar.total, 256);
-    COLA_CUDA(cudaMalloc(&g->dmem, ar.total));
+    COLA_CUDA(device_alloc(&g->dmem, ar.total));
     g->dbytes = ar.total;
     char *base = static_cast<char *>(g->dmem);
     auto at = [&](size_t o) { return reinterpret_cast<const int32_t *>(base + o); };

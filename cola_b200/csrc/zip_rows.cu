@@ -131,7 +131,7 @@ static cola_status build(const cola_zip_part *parts, int32_t nparts, const int64
     void *arena = nullptr;
     const size_t a = 256, n = (size_t)std::max<int64_t>(nnz, 1);
     const size_t slice = (4 * n + a - 1) / a * a;
-    COLA_CUDA(cudaMallocAsync(&arena, 3 * slice + a, st));
+    COLA_CUDA(scratch_alloc(&arena, 3 * slice + a, st));
     char *base = static_cast<char *>(arena);
     int32_t *row = reinterpret_cast<int32_t *>(base);
     int32_t *col = reinterpret_cast<int32_t *>(base + slice);

@@ -418,6 +418,11 @@ cola_status cola_probe_gather(int64_t table_bytes, int32_t row_bytes, int64_t ga
 cola_status cola_probe_graph_gather(const cola_graph *g, const void *X, int64_t ld_bytes, int32_t row_bytes,
                                     int32_t reps, cola_stream_t stream, double *gbps, float *ms_per_pass);
 
+/* Gives the device memory the library keeps for reuse (up to 1 GiB per device,
+ * freed by earlier builds and graphs) back to the device; waits for the current
+ * device. */
+cola_status cola_trim_memory(void);
+
 /* Waits for the current device, then reports (and clears) the error code a
  * kernel left when one of its bounded waits ran out: 0 = none; 1 = a bulk-copy
  * gather stopped early (it drained every copy it had issued before exiting);
