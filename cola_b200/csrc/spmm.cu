@@ -447,7 +447,7 @@ static cola_status launch_block_t(const dev::BlockArgs &ba, const RowsLaunch &a,
     auto fn = dyn ? dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, true>
                   : dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, false>;
     t_launches++;
-    COLA_CUDA(launch_kernel(fn, (unsigned)grid_for((const void *)fn, ba.nitem), (unsigned)ntile, false, st, ba,
+    COLA_CUDA(launch_kernel(fn, (unsigned)grid_for((const void *)fn, ba.nitem), (unsigned)ntile, true, st, ba,
                             static_cast<const T *>(a.X), a.ldx, static_cast<TY *>(a.Y), a.ldy, a.K, a.accumulate));
     return COLA_SUCCESS;
 }
@@ -463,7 +463,7 @@ static cola_status launch_block_odd_t(const dev::BlockArgs &ba, const RowsLaunch
     auto fn = dyn ? dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, true, false>
                   : dev::rowblock_spmm_kernel<TR, TY, LG, NV, UNROLL, MINB, false, false>;
     t_launches++;
-    COLA_CUDA(launch_kernel(fn, (unsigned)grid_for((const void *)fn, ba.nitem), (unsigned)ntile, false, st, ba,
+    COLA_CUDA(launch_kernel(fn, (unsigned)grid_for((const void *)fn, ba.nitem), (unsigned)ntile, true, st, ba,
                             static_cast<const T *>(a.X), a.ldx, static_cast<TY *>(a.Y), a.ldy, a.K, a.accumulate));
     return COLA_SUCCESS;
 }

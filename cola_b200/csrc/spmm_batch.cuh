@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kThreads, MINB) batch_rowblock_kernel(const Ba
         for (int k0 = 0; k0 < bg.K; k0 += W) {
             RowStream<TR, TY, LG, NV, UNROLL> rs;
             rs.init(static_cast<const T *>(bg.X), bg.ldx, static_cast<TY *>(bg.Y), bg.ldy, bg.K, k0, accumulate);
-            stream_item(rs, bg.ba, li, eb);
+            stream_item(rs, bg.ba, li, eb, []() {});
         }
         it = draw ? __shfl_sync(kFull, next, 0) : it + nwarps;
     }

@@ -565,10 +565,17 @@ struct RowStream {
     }
 };
 
+// Programmatic dependent launch: the next kernel's blocks may start once every
+// block of this grid has said so or ended; they wait for this grid's end, and so
+// for all that was before it, with pdl_wait.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // One work item.  While a batch is summed the next one's entries are on their
-// way in registers.
-template <typename RS>
-__device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const int it, EntryBatch &eb)
+// way in registers.  before_x() runs when the first entries are under way and
+// before X is read or anything written.
+template <typename RS, typename F>
+__device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const int it, EntryBatch &eb, F before_x)
 {
     const int lane = rs.lane;
     const bool seg = it < ba.nseg;
@@ -589,6 +596,7 @@ __device__ __forceinline__ void stream_item(RS &rs, const BlockArgs &ba, const i
             mr = __ldg(ba.nz_row + kpos);  // the list is padded by 32
     };
     fetch();
+    before_x();
     rs.clear();
     while (left > 0) {
         const int n = min(32, left);
@@ -633,7 +641,9 @@ __device__ __forceinline__ unsigned int draw_item(unsigned int *queue, unsigned 
 }
 
 // All items of one feature tile, drawn by this warp, one ahead, so that the
-// atomic's latency hides behind the current item.
+// atomic's latency hides behind the current item.  The grid may have started
+// before the kernel in front of it has ended: only the graph's own arrays, which
+// no kernel writes, are read before pdl_wait.
 template <typename RS, bool DYN>
 __device__ __forceinline__ void stream_items(RS &rs, const BlockArgs &ba, const unsigned int warp,
                                              const unsigned int nwarps, EntryBatch &eb,
@@ -644,9 +654,12 @@ __device__ __forceinline__ void stream_items(RS &rs, const BlockArgs &ba, const 
     const bool draw = DYN && total > nwarps;
     for (unsigned int it = warp; it < total;) {
         unsigned int next = DYN ? total : it + nwarps;
-        if (draw && rs.lane == 0)
-            next = draw_item(queue, nwarps);
-        stream_item(rs, ba, (int)it, eb);
+        stream_item(rs, ba, (int)it, eb, [&]() {
+            if (it == warp)
+                pdl_wait();
+            if (draw && rs.lane == 0)
+                next = draw_item(queue, nwarps);
+        });
         it = draw ? __shfl_sync(kFull, next, 0) : next;
     }
 }
@@ -665,11 +678,6 @@ __device__ __forceinline__ void item_queue_release(unsigned int *queue, const un
         }
     }
 }
-
-// Launch of a dependent kernel may begin (its blocks wait for this grid's end
-// with pdl_wait): every block of these grids is resident when it says so.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB = 1, bool DYN = false, bool VEC_Y = true>
 __global__ void __launch_bounds__(kThreads, MINB) rowblock_spmm_kernel(const __grid_constant__ BlockArgs ba,
@@ -922,6 +930,7 @@ __global__ void __launch_bounds__(kThreads, 3) hub_combine_vec_kernel(const int3
                                                                   float *ws, int64_t ld_ws, TY *__restrict__ Y,
                                                                   int64_t ldy, int K, int accumulate)
 {
+    pdl_launch_dependents();
     pdl_wait();  // the partials
     const int tiles = hub_tiles(K);
     hub_combine_all<TY, VEC_Y>(nhub * tiles, hub_lanes(K), accumulate, [&](int64_t w) {

@@ -16,8 +16,15 @@ from ._lib import (BFLOAT16, FLOAT32, SCHEDULE_AUTO, SCHEDULE_BUFFER, SCHEDULE_F
 _DT = {torch.float32: FLOAT32, torch.bfloat16: BFLOAT16}
 
 
+# torch.cuda.current_stream() builds a Stream object, 3.4 us of an 11 us spmm()
+# call; this reads the same handle
+_current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream):
     if stream is None:
+        if _current_raw_stream is not None:
+            return ctypes.c_void_p(_current_raw_stream(torch.cuda.current_device()))
         return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
     if isinstance(stream, torch.cuda.Stream):
         return ctypes.c_void_p(stream.cuda_stream)
@@ -116,15 +123,10 @@ class Graph:
         _dense(Y, "Y")
         if Y.shape[0] < self.num_nodes or Y.shape[1] != K:
             raise ValueError("Y must be {} x {}".format(self.num_nodes, K))
-        o = SpmmOpts()
-        o.accumulate = 1 if accumulate else 0
-        o.schedule = int(schedule)
-        o.gather_batch_rows = int(gather_batch_rows)
-        o.unroll = int(unroll)
-        o.min_blocks = int(min_blocks)
-        o.k_tile = int(k_tile)
-        check(lib().cola_spmm(self._h, _ptr(X), _DT[X.dtype], X.stride(0), _ptr(Y), _DT[Y.dtype], Y.stride(0), K,
-                              ctypes.byref(o), _stream(stream)))
+        o = SpmmOpts(1 if accumulate else 0, int(schedule), int(gather_batch_rows), int(unroll), int(min_blocks),
+                     int(k_tile))
+        check(lib().cola_spmm(self._h, X.data_ptr(), _DT[X.dtype], X.stride(0), Y.data_ptr(), _DT[Y.dtype],
+                              Y.stride(0), K, ctypes.byref(o), _stream(stream)))
         return Y
 
     def spmm_host(self, X, Y, schedule=SCHEDULE_AUTO, stream=None):
