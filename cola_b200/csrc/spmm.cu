@@ -1513,10 +1513,12 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
     }
 
     if (ydt == COLA_BFLOAT16) {
-        const int64_t n = (int64_t)g->N * K;
+        const bool vec = K % 4 == 0 && ldacc % 4 == 0 && ldy % 4 == 0 && aligned16(acc) && ((uintptr_t)Y & 7u) == 0;
+        const int64_t n = (int64_t)g->N * K / (vec ? 4 : 1);
         const int64_t blocks = std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 8);
         t_launches++;
-        dev::f32_to_bf16_kernel<<<(unsigned)std::max<int64_t>(blocks, 1), dev::kThreads, 0, st>>>(
+        auto fn = vec ? dev::f32_to_bf16_kernel<4> : dev::f32_to_bf16_kernel<1>;
+        fn<<<(unsigned)std::max<int64_t>(blocks, 1), dev::kThreads, 0, st>>>(
             acc, ldacc, static_cast<__nv_bfloat16 *>(Y), ldy, g->N, K);
         COLA_CUDA(cudaGetLastError());
     }

