@@ -37,12 +37,13 @@ __global__ void __launch_bounds__(kThreads, MINB) batch_rowblock_kernel(const Ba
     using T = typename ElemOf<TR>::T;
     __shared__ EntryBatch s_ent[kWarpsPerBlock];
     pdl_launch_dependents();
-    EntryBatch &eb = s_ent[threadIdx.x >> 5];
+    const unsigned int wb = warp_in_block();
+    EntryBatch &eb = s_ent[wb];
     const unsigned int nwarps = gridDim.x * kWarpsPerBlock;
-    const int lane = threadIdx.x & 31;
+    const int lane = lane_id();
     const bool draw = DYN && total > nwarps;
     int gi = 0;
-    unsigned int it = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    unsigned int it = blockIdx.x * kWarpsPerBlock + wb;
     while (it < total) {
         unsigned int next = 0;
         if (draw && lane == 0)

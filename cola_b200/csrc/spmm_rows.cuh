@@ -306,13 +306,19 @@ __device__ __forceinline__ const char *row_at(const char *base, int32_t c, int32
     return reinterpret_cast<const char *>(r);
 }
 
-// Lane id as a value the compiler keeps (it re-reads threadIdx, a slow special
-// register, inside the loops otherwise).
+// Lane id and warp in the block as values the compiler keeps (it re-reads
+// threadIdx, a slow special register, inside the loops otherwise).
 __device__ __forceinline__ int lane_id()
 {
     int l;
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
     return l;
+}
+__device__ __forceinline__ unsigned int warp_in_block()
+{
+    unsigned int t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t >> 5;
 }
 
 // How an item's entries are summed: LG lanes cover one row tile of X (NV
@@ -538,6 +544,51 @@ struct RowStream {
                     if (e & (1u << u))
                         flush();
                 }
+            } else if constexpr (G == 2 && E <= 4 && UNROLL <= 4) {
+                // pair by pair: a row ends after the first or the second of a pair
+#pragma unroll
+                for (int u = 0; u < UNROLL; u++) {
+                    const uint32_t p = (e >> (2 * u)) & 3u;
+                    const bool have = 2 * u + g < cnt;
+                    auto add = [&]() {
+#pragma unroll
+                        for (int j = 0; j < NV; j++)
+                            fma_vec2<TR>(acc[j], v[u], xr[u][j]);
+                    };
+                    if (have && (g == 0 || !(p & 1u)))
+                        add();
+                    if (p & 1u) {
+                        flush();
+                        if (have && g == 1)
+                            add();
+                    }
+                    if (p & 2u)
+                        flush();
+                }
+            } else if constexpr (G > 1 && UNROLL > 1) {
+                // one entry per group at a time, cut where rows end among them
+#pragma unroll
+                for (int u = 0; u < UNROLL; u++) {
+                    uint32_t p = (e >> (u * G)) & ((1u << G) - 1u);
+                    const bool have = u * G + g < cnt;
+                    int lo = 0;
+                    while (p) {
+                        const int sh = __ffs(p);
+                        if (have && g >= lo && g < sh) {
+#pragma unroll
+                            for (int j = 0; j < NV; j++)
+                                fma_vec2<TR>(acc[j], v[u], xr[u][j]);
+                        }
+                        flush();
+                        p &= p - 1;
+                        lo = sh;
+                    }
+                    if (have && g >= lo) {
+#pragma unroll
+                        for (int j = 0; j < NV; j++)
+                            fma_vec2<TR>(acc[j], v[u], xr[u][j]);
+                    }
+                }
             } else {
                 // cut the round at the row ends it contains
                 int lo = 0;
@@ -689,11 +740,10 @@ __global__ void __launch_bounds__(kThreads, MINB) rowblock_spmm_kernel(const __g
     pdl_launch_dependents();
     constexpr int W = LG * NV * TR::E;
     const int k0 = blockIdx.y * W;
-    const unsigned int nwarps = gridDim.x * kWarpsPerBlock;
+    const unsigned int nwarps = gridDim.x * kWarpsPerBlock, wb = warp_in_block();
     RowStream<TR, TY, LG, NV, UNROLL, VEC_Y> rs;
     rs.init(X, ldx, Y, ldy, K, k0, accumulate);
-    stream_items<RowStream<TR, TY, LG, NV, UNROLL, VEC_Y>, DYN>(rs, ba, blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5),
-                                                         nwarps, s_ent[threadIdx.x >> 5],
+    stream_items<RowStream<TR, TY, LG, NV, UNROLL, VEC_Y>, DYN>(rs, ba, blockIdx.x * kWarpsPerBlock + wb, nwarps, s_ent[wb],
                                                          DYN ? ba.queue + blockIdx.y : nullptr);
     if (DYN && (unsigned int)ba.nitem > nwarps)
         item_queue_release(ba.queue, gridDim.y, ba.queue + kMaxItemQueues, nwarps * gridDim.y);
