@@ -100,10 +100,8 @@ static cola_status launch_fused_t(const FusedArgs &a, cudaStream_t st)
     const int64_t gx = std::max<int64_t>(1, (a.total + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
     const int gy = (a.K + W - 1) / W;
     t_launches++;
-    fn<<<dim3((unsigned)gx, (unsigned)gy), dev::kThreads, 0, st>>>(a.parts, a.single, a.nparts, a.total,
-                                                                   static_cast<const T *>(a.X), a.ldx, a.Y, a.ldy,
-                                                                   a.K);
-    COLA_CUDA(cudaGetLastError());
+    COLA_CUDA(launch_kernel(fn, (unsigned)gx, (unsigned)gy, true, st, a.parts, a.single, a.nparts, a.total,
+                            static_cast<const T *>(a.X), a.ldx, a.Y, a.ldy, a.K));
     return COLA_SUCCESS;
 }
 
@@ -161,9 +159,8 @@ static cola_status launch_stream_t(const FusedArgs &a, cudaStream_t st)
     const int span = kFusedSpan;
     const int64_t gx = (a.total + (int64_t)span * dev::kWarpsPerBlock - 1) / ((int64_t)span * dev::kWarpsPerBlock);
     t_launches++;
-    fn<<<dim3((unsigned)gx, (unsigned)((a.K + W - 1) / W)), dev::kThreads, 0, st>>>(
-        a.parts, a.single, a.nparts, a.total, span, static_cast<const T *>(a.X), a.ldx, a.Y, a.ldy, a.K);
-    COLA_CUDA(cudaGetLastError());
+    COLA_CUDA(launch_kernel(fn, (unsigned)gx, (unsigned)((a.K + W - 1) / W), true, st, a.parts, a.single, a.nparts,
+                            a.total, span, static_cast<const T *>(a.X), a.ldx, a.Y, a.ldy, a.K));
     return COLA_SUCCESS;
 }
 

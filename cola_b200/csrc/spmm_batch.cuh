@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kThreads, MINB) batch_rowblock_kernel(const Ba
 }
 
 template <typename TY>
-__global__ void __launch_bounds__(kThreads, 3) batch_hub_combine_kernel(const BatchGraph *__restrict__ gs, int ng,
+__global__ void __launch_bounds__(kThreads, 4) batch_hub_combine_kernel(const BatchGraph *__restrict__ gs, int ng,
                                                                     int64_t total, int lanes, int accumulate)
 {
     pdl_wait();  // the partials

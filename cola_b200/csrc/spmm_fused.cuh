@@ -188,6 +188,8 @@ __global__ void __launch_bounds__(kThreads, MINB) fused_stream_kernel(const Part
                                                                 int64_t ldx, float *__restrict__ Y, int64_t ldy, int K)
 {
     __shared__ EntryBatch s_ent[kWarpsPerBlock];
+    pdl_launch_dependents();
+    pdl_wait();
     EntryBatch &eb = s_ent[threadIdx.x >> 5];
     const int k0 = blockIdx.y * (LG * NV * TR::E);
     const int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);

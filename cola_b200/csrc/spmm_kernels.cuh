@@ -31,6 +31,12 @@ constexpr int32_t kColMask = INT32_MAX;
 // Padding of the list of rows with entries (read 32 at a time).
 constexpr int kRowPad = 32;
 
+// Programmatic dependent launch: the next kernel's blocks may start once every
+// block of this grid has said so or ended; they wait for this grid's end, and so
+// for all that was before it, with pdl_wait.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Where a remote chunk's dense row comes from.
 enum RemoteMode : int32_t {
     kRemoteFromX = 0,       // X[x_remote0 + global col]           (on-chip staging)
@@ -225,6 +231,8 @@ __global__ void __launch_bounds__(kThreads, MINB) fused_spmm_kernel(const PartDe
                                                               const typename ElemOf<TR>::T *__restrict__ X,
                                                               int64_t ldx, float *__restrict__ Y, int64_t ldy, int K)
 {
+    pdl_launch_dependents();
+    pdl_wait();  // the chunks too may come from the kernel before
     using T = typename ElemOf<TR>::T;
     using raw_t = typename TR::raw_t;
     constexpr int E = TR::E;

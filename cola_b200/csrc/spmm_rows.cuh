@@ -616,12 +616,6 @@ struct RowStream {
     }
 };
 
-// Programmatic dependent launch: the next kernel's blocks may start once every
-// block of this grid has said so or ended; they wait for this grid's end, and so
-// for all that was before it, with pdl_wait.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // One work item.  While a batch is summed the next one's entries are on their
 // way in registers.  before_x() runs when the first entries are under way and
 // before X is read or anything written.
@@ -975,7 +969,7 @@ __device__ __forceinline__ void hub_combine_all(const int64_t total, const int l
 }
 
 template <typename TY, bool VEC_Y>
-__global__ void __launch_bounds__(kThreads, 3) hub_combine_vec_kernel(const int32_t *__restrict__ hub_row,
+__global__ void __launch_bounds__(kThreads, 4) hub_combine_vec_kernel(const int32_t *__restrict__ hub_row,
                                                                   const int64_t *__restrict__ hub_seg, int64_t nhub,
                                                                   float *ws, int64_t ld_ws, TY *__restrict__ Y,
                                                                   int64_t ldy, int K, int accumulate)
