@@ -63,11 +63,12 @@ inline unsigned hub_blocks(int64_t items, int lanes)
     return (unsigned)(need < 1 ? 1 : need < most ? need : most);
 }
 // Device memory (memory.cu).  device_alloc: usable on every stream when it
-// returns; device_free: waits for the device first.  scratch_alloc: ordered on
-// `st` (cudaFreeAsync gives it back).
+// returns; device_free: waits for the device first.  scratch_alloc and
+// scratch_free (the same bytes): ordered on `st`.
 cudaError_t device_alloc(void **p, size_t bytes);
 void device_free(void *p);
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
+void scratch_free(void *p, size_t bytes, cudaStream_t st);
 // Grow a device allocation to at least `need` bytes (contents not kept).
 cola_status ensure(void *&p, size_t &have, size_t need);
 

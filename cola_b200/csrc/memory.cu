@@ -3,7 +3,7 @@
 // about 7 ms a gigabyte each with the default pool (which unmaps at every
 // synchronisation) and 0.5 ms or more per cudaMalloc or cudaFree, most of the
 // wall time of building a graph (1 M rows, 14 M entries, and one SpMM: 4.8 ms and
-// up to 29 on a busy host, 1.84 with the pool).  The kept bytes are given back by
+// up to 29 on a busy host, 1.8 with the pool).  The kept bytes are given back by
 // cola_trim_memory and before the library reports that the device is full; the
 // driver gives back what exceeds kKeep at each synchronisation.  Pools are safe
 // with several threads and streams: memory freed on one stream is handed to
@@ -66,9 +66,22 @@ static void trim(const DevicePool &p)
     cudaGetLastError();
 }
 
+// Requests past kPooled go to cudaMalloc and cudaFree: about 1 ms each at 700 MB,
+// where the pool, which keeps no more than kKeep, would map and unmap for 10.
+constexpr size_t kPooled = kKeep / 2;
+
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st)
 {
     const DevicePool dp = device_pool_entry();
+    if (bytes > kPooled) {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            trim(dp);
+            e = cudaMalloc(p, bytes);
+        }
+        return e;
+    }
     if (!dp.pool)
         return cudaMallocAsync(p, bytes, st);
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, dp.pool, st);
@@ -80,10 +93,20 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st)
     return e;
 }
 
+void scratch_free(void *p, size_t bytes, cudaStream_t st)
+{
+    if (bytes > kPooled) {
+        cudaStreamSynchronize(st);
+        cudaFree(p);
+    } else {
+        cudaFreeAsync(p, st);
+    }
+}
+
 cudaError_t device_alloc(void **p, size_t bytes)
 {
     const DevicePool dp = device_pool_entry();
-    if (dp.pool) {
+    if (dp.pool && bytes <= kPooled) {
         if (cudaMallocFromPoolAsync(p, bytes, dp.pool, dp.stream) == cudaSuccess) {
             const cudaError_t e = cudaStreamSynchronize(dp.stream);  // usable on every stream from here on
             if (e != cudaSuccess)
@@ -91,17 +114,27 @@ cudaError_t device_alloc(void **p, size_t bytes)
             return e;
         }
         cudaGetLastError();
-        trim(dp);
     }
-    return cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && dp.pool) {
+        cudaGetLastError();
+        trim(dp);
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 void device_free(void *p)
 {
     if (!p)
         return;
-    // cudaFree waits for the device itself only for memory from cudaMalloc
-    cudaDeviceSynchronize();
+    // cudaFree waits for the device itself only for memory from cudaMalloc; where
+    // that wait is refused (a stream is being captured) the memory stays, as it
+    // would with cudaFree
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
     cudaFree(p);
 }
 

@@ -253,8 +253,8 @@ __global__ void __launch_bounds__(kThreads) radix_hist_kernel(const uint64_t *ke
 // tile by digit in shared memory, so that each digit's entries are written as
 // one run.  Bound by HBM (24 bytes per entry).  Writing every entry straight to
 // its place, with two block-wide waits per 256 entries, took 0.28 ms per digit
-// of a 14 M-entry sort, the counts 0.095; now 0.14 and 0.06.
-__global__ void __launch_bounds__(kThreads) radix_scatter_kernel(const uint64_t *kin, const float *vin,
+// of a 14 M-entry sort, the counts 0.095; now 0.11 and 0.06.
+__global__ void __launch_bounds__(kThreads, 3) radix_scatter_kernel(const uint64_t *kin, const float *vin,
                                                                  uint64_t *kout, float *vout, int64_t n, int shift,
                                                                  int64_t ntiles, const uint32_t *hist_scan)
 {
@@ -266,15 +266,12 @@ __global__ void __launch_bounds__(kThreads) radix_scatter_kernel(const uint64_t 
     const int64_t tile0 = (int64_t)blockIdx.x * kTile;
     const int cnt = (int)min((int64_t)kTile, n - tile0);
     uint64_t k[kItems];
-    float v[kItems];
     uint32_t rk[kItems];
     const int at0 = w * (kItems * 32) + lane;
 #pragma unroll
     for (int r = 0; r < kItems; r++)
-        if (at0 + r * 32 < cnt) {
+        if (at0 + r * 32 < cnt)
             k[r] = kin[tile0 + at0 + r * 32];
-            v[r] = vin[tile0 + at0 + r * 32];
-        }
     for (int b = lane; b < kBins; b += 32)
         wcnt[w][b] = 0;
     __syncwarp();
@@ -313,6 +310,11 @@ __global__ void __launch_bounds__(kThreads) radix_scatter_kernel(const uint64_t 
             sk[rk[r]] = k[r];
         }
     __syncthreads();
+    float v[kItems];  // under way while the keys are written
+#pragma unroll
+    for (int r = 0; r < kItems; r++)
+        if (at0 + r * 32 < cnt)
+            v[r] = vin[tile0 + at0 + r * 32];
     uint32_t pos[kItems];
 #pragma unroll
     for (int r = 0; r < kItems; r++) {
@@ -748,14 +750,14 @@ inline unsigned grid_stride_blocks(int64_t n)
 // for the whole call), else one stream-ordered allocation per request.
 struct Scratch {
     cudaStream_t st;
-    std::vector<void *> ptrs;
+    std::vector<std::pair<void *, size_t>> ptrs;
     char *arena = nullptr;
     size_t used = 0, cap = 0;
     explicit Scratch(cudaStream_t s) : st(s) {}
     ~Scratch()
     {
-        for (void *p : ptrs)
-            cudaFreeAsync(p, st);
+        for (const auto &p : ptrs)
+            scratch_free(p.first, p.second, st);
     }
     cola_status alloc(void *&q, size_t bytes)
     {
@@ -763,7 +765,7 @@ struct Scratch {
         if (e != cudaSuccess)
             return fail(e == cudaErrorMemoryAllocation ? COLA_ERROR_OUT_OF_MEMORY : COLA_ERROR_CUDA,
                         "device preprocessing: %zu bytes: %s", bytes, cudaGetErrorString(e));
-        ptrs.push_back(q);
+        ptrs.push_back({q, bytes});
         return COLA_SUCCESS;
     }
     cola_status reserve(size_t bytes)

@@ -180,7 +180,7 @@ static cola_status build(const cola_zip_part *parts, int32_t nparts, const int64
         const int64_t ncols = std::max<int64_t>(nrows, nnz > 0 ? (int64_t)h_mx[1] + 1 : 0);
         rc = graph_build_device_rect((int32_t)nrows, (int32_t)ncols, nnz, row, col, val, nullptr, st, g, who);
     }
-    cudaFreeAsync(arena, st);
+    scratch_free(arena, 3 * slice + a, st);
     if (rc != COLA_SUCCESS)
         return rc;
     cola_zip_rows *h = new (std::nothrow) cola_zip_rows();
