@@ -403,23 +403,17 @@ static cola_status launch_rows_geo(const RowsLaunch &a, int V, cudaStream_t st)
     return launch_rows_t<TR, TY, 32, 4, 2, VEC>(a, st);
 }
 
+// Element by element (pad_x says when).
 static cola_status launch_rows(const RowsLaunch &a, cudaStream_t st)
 {
     if (a.ra.nseg + a.ra.nrows <= 0 || a.K <= 0)
         return COLA_SUCCESS;
     using BF = __nv_bfloat16;
-    if (a.xdt == COLA_FLOAT32) {
-        if (a.ydt == COLA_FLOAT32)
-            return a.vec ? launch_rows_geo<dev::VecTraits<float>, float, true>(a, a.K / 4, st)
-                         : launch_rows_geo<dev::ScalarTraits<float>, float, false>(a, a.K, st);
-        return a.vec ? launch_rows_geo<dev::VecTraits<float>, BF, true>(a, a.K / 4, st)
-                     : launch_rows_geo<dev::ScalarTraits<float>, BF, false>(a, a.K, st);
-    }
-    if (a.ydt == COLA_FLOAT32)
-        return a.vec ? launch_rows_geo<dev::VecTraits<BF>, float, true>(a, a.K / 8, st)
-                     : launch_rows_geo<dev::ScalarTraits<BF>, float, false>(a, a.K, st);
-    return a.vec ? launch_rows_geo<dev::VecTraits<BF>, BF, true>(a, a.K / 8, st)
-                 : launch_rows_geo<dev::ScalarTraits<BF>, BF, false>(a, a.K, st);
+    if (a.xdt == COLA_FLOAT32)
+        return a.ydt == COLA_FLOAT32 ? launch_rows_geo<dev::ScalarTraits<float>, float, false>(a, a.K, st)
+                                     : launch_rows_geo<dev::ScalarTraits<float>, BF, false>(a, a.K, st);
+    return a.ydt == COLA_FLOAT32 ? launch_rows_geo<dev::ScalarTraits<BF>, float, false>(a, a.K, st)
+                                 : launch_rows_geo<dev::ScalarTraits<BF>, BF, false>(a, a.K, st);
 }
 
 template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB = 1>
@@ -553,7 +547,8 @@ static cola_status launch_block_geo(const dev::BlockArgs &ba, const RowsLaunch &
     return launch_block_t<TR, TY, 32, 2, 4, 3>(ba, a, st);
 }
 
-// Feature tile of one pass for the requested k_tile (0 = the library's
+// Feature tile of one pass (at most two vectors a lane: 256 FP32 or 512 BF16
+// features, wider requests run as that) for the requested k_tile (0 = the library's
 // choice), in the regime where a full warp covers one tile (K >= 128 FP32 X,
 // K >= 256 BF16 X); 0 where k_tile does not apply.
 static int rows_k_tile(cola_dtype xdt, int K, int k_tile)
