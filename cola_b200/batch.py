@@ -1,5 +1,5 @@
 """Batched form: many graphs, each with its own X, Y and feature width, in one
-persistent launch (plus one for hub rows), capturable in a CUDA graph, with the
+persistent launch per lane width (plus one for hub rows), capturable in a CUDA graph, with the
 project's launch-parameter autotuner.  Backed by the cola_batch_* C ABI."""
 import ctypes
 import os

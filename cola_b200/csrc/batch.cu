@@ -1,6 +1,6 @@
 // Batched form of the partitioned SpMM: many graphs of uneven size, each with
-// its own dense operands and feature width, in one persistent launch (plus one
-// for hub rows), capturable in a CUDA graph; and the launch-parameter autotuner.
+// its own dense operands and feature width, in one persistent launch per lane
+// width (plus one for hub rows), capturable in a CUDA graph; and the launch-parameter autotuner.
 #include <algorithm>
 #include <climits>
 #include <cstdio>

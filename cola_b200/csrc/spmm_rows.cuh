@@ -335,7 +335,7 @@ __device__ __forceinline__ unsigned int warp_in_block()
 // Measured (R-MAT, one lane group a row): scale 20, K = 128 FP32 1.11 -> 1.07 ms
 // against the form that walked row pointers, scale 21, K = 256 BF16 4.03 ->
 // 3.85, uniform rows of 20 entries at K = 100 83 -> 74 us; narrow rows: K = 16
-// BF16 206 -> 126 us, K = 32 FP32 on 16 K rows 23 -> 14 us.  Slower: 8 rows in
+// BF16 206 -> 117 us, K = 32 FP32 on 16 K rows 23 -> 13 us.  Slower: 8 rows in
 // flight at 3 blocks (1.10 ms), 2 at 5 or 6 (1.35), the next row's load issued
 // as each row is added (1.64).
 // VEC_Y: rows of Y are written in vectors; else (their start is not aligned or K
@@ -812,7 +812,10 @@ __global__ void __launch_bounds__(kThreads) hub_combine_kernel(const int32_t *__
 // those to kHubRadix^2, and so on; then the open blocks of every power are
 // folded.  Hubs of kHubTeam or more partials are left to the end and each shared
 // by the whole block: one lane group alone walks 240 partials in 55 us, which
-// was the tail of the launch.
+// was the tail of the launch.  Measured in the step, launch included: 16 K rows
+// at K = 32 6.7 -> 2.6 us, 524 K rows at K = 16 27 -> 10, scale 20 at K = 128
+// 56 -> 33.  Teams from 32 partials on: below, one group's few rounds cost less
+// than the block's waits.
 constexpr int kHubRadixBits = 3, kHubRadix = 1 << kHubRadixBits;
 constexpr int kHubTeam = 32;
 constexpr int kHubList = 128;  // long hubs a block keeps for its end; more are walked alone

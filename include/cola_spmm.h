@@ -518,7 +518,8 @@ cola_status cola_spmm_host_join(cola_graph *g, cola_stream_t stream);
 
 /* ========================================================================
  * Batched form: many graphs of uneven size, each with its own X, Y and
- * feature width, in one persistent launch (plus one for hub rows).
+ * feature width, in one persistent launch per lane width (how many lanes a
+ * row's vectors take; the launches overlap) plus one for hub rows.
  * ====================================================================== */
 
 typedef struct cola_batch cola_batch;
@@ -529,8 +530,7 @@ cola_status cola_batch_create(const cola_partition_set *const *parts, int32_t ng
                               cola_batch **out, cola_stream_t stream);
 /* A batch over graphs that already exist (cola_graph_upload with the row
  * view, or cola_graph_build_device).  The batch borrows them (free the batch
- * first, then the graphs) and uses each graph's hub workspace, so a graph of
- * the batch must not run elsewhere while the batch runs. */
+ * first, then the graphs) and keeps a hub workspace of its own. */
 cola_status cola_batch_create_from_graphs(cola_graph *const *graphs, int32_t ngraphs, cola_batch **out);
 cola_status cola_batch_free(cola_batch *b);
 
@@ -553,9 +553,10 @@ cola_status cola_batch_run(cola_batch *b, const cola_spmm_opts *opts, cola_strea
 cola_status cola_batch_capture(cola_batch *b, const cola_spmm_opts *opts, cola_stream_t stream);
 cola_status cola_batch_replay(cola_batch *b, cola_stream_t stream);
 
-/* Launch parameters of the batched kernel: loads in flight per lane group (2
- * or 4), the persistent grid as a percentage of one full wave and the resident
- * blocks per SM it is compiled for (3 or 4). */
+/* Launch parameters of the batched kernel (graphs whose rows take a full warp;
+ * narrower ones have one geometry): loads in flight per lane group (2 or 4),
+ * the persistent grid as a percentage of one full wave and the resident blocks
+ * per SM it is compiled for (3 or 4). */
 cola_status cola_batch_set_params(cola_batch *b, int32_t unroll, int32_t grid_pct, int32_t blocks_per_sm);
 
 /* The project's autotuner for the batched launch: times every candidate
