@@ -63,7 +63,8 @@ inline unsigned hub_blocks(int64_t items, int lanes)
     return (unsigned)(need < 1 ? 1 : need < most ? need : most);
 }
 // Device memory (memory.cu).  device_alloc: usable on every stream when it
-// returns; device_free: waits for the device first.  scratch_alloc and
+// returns; device_free: waits for the device first; both may be called while a
+// stream is being captured, by this thread or another.  scratch_alloc and
 // scratch_free (the same bytes): ordered on `st`.
 cudaError_t device_alloc(void **p, size_t bytes);
 void device_free(void *p);
