@@ -2,6 +2,7 @@
 // translation units of the library (not part of the C ABI).
 #pragma once
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -79,6 +80,31 @@ using cola::dev::GatherSeg;
 using cola::dev::PartDesc;
 
 namespace cola {
+// A device workspace of a graph; grows, see grow().
+struct Workspace {
+    void *p = nullptr;
+    size_t bytes = 0;
+    bool captured = false;  // a captured call names it: it lives as long as its owner
+    float *f() const { return static_cast<float *>(p); }
+};
+// The workspaces that grew after a captured call had named them: replays of that
+// call still use them.
+struct KeptBlocks {
+    std::vector<std::pair<void *, size_t>> blocks;
+    size_t bytes() const
+    {
+        size_t n = 0;
+        for (const auto &b : blocks)
+            n += b.second;
+        return n;
+    }
+};
+// Whether work put on `st` now is recorded instead of run.
+bool is_capturing(cudaStream_t st);
+// At least `need` bytes in w for a call on a stream that is being captured or
+// not; the contents are not kept, the old block is if a captured call names it.
+cola_status grow(Workspace &w, size_t need, bool capturing, KeptBlocks &kept);
+
 struct HostPipe;  // cola_spmm_host's staging sets and copy streams
 void host_pipe_release(HostPipe *p);
 }  // namespace cola
@@ -106,12 +132,10 @@ struct cola_graph {
     std::vector<int64_t> put_total;
     std::vector<std::vector<GatherSeg>> h_put;
     // lazily sized workspaces
-    void *ppl_buf = nullptr;  // 2 x P x npp x K elements
-    size_t ppl_bytes = 0;
-    void *stage_buf = nullptr;  // BUFFER schedule staging
-    size_t stage_bytes = 0;
-    float *ws = nullptr;  // FP32 accumulator for BF16 output
-    size_t ws_bytes = 0;
+    cola::Workspace ppl_buf;    // 2 x P x npp x K elements
+    cola::Workspace stage_buf;  // BUFFER schedule staging
+    cola::Workspace ws;         // FP32 accumulator for BF16 output
+    cola::KeptBlocks kept;
     int64_t last_launches = 0;       // kernels launched by the last cola_spmm call
     GatherSeg *d_bufsegs = nullptr;  // BUFFER schedule gather segments
     std::vector<GatherSeg> h_bufsegs;
@@ -131,13 +155,11 @@ struct cola_graph {
     const int32_t *nz_row = nullptr, *empty_row = nullptr;
     int64_t nseg = 0, nhub = 0, ntask = 0, nempty = 0;
     int32_t hub_threshold = 256, hub_segment = 256, task_entries = 128;
-    float *ws_hub = nullptr;  // nseg x K partials
+    cola::Workspace ws_hub;  // nseg x K partials
     // dev::kMaxItemQueues + 1 work-item counters of the row-major schedule,
     // in dmem, zero between launches
     unsigned int *item_queue = nullptr;
-    size_t ws_hub_bytes = 0;
-    void *x_pad = nullptr;  // X with padded rows (widths no vector divides)
-    size_t x_pad_bytes = 0;
+    cola::Workspace x_pad;  // X with padded rows (widths no vector divides)
     cola::HostPipe *host_pipe = nullptr;  // created by the first cola_spmm_host call
 };
 

@@ -616,7 +616,7 @@ bool vec_ok_rows(cola_dtype xdt, const void *X, int64_t ldx, cola_dtype ydt, con
 // has no room for it.  The scalar kernel remains for those calls.  K = 33 FP32,
 // 150 K rows, 2.4 M entries: 185 -> 73 us, K = 74 BF16 209 -> 100, K = 301 FP32
 // 717 -> 337, K = 33 at 3 entries a row 86 -> 42.
-static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool &x_ok, cudaStream_t st)
+static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool &x_ok, bool capturing, cudaStream_t st)
 {
     const int E = a.xdt == COLA_FLOAT32 ? 4 : 8, esz = 16 / E;
     x_ok = a.K % E == 0 && a.ldx % E == 0 && a.ldx <= INT32_MAX / esz && aligned16(a.X);
@@ -624,16 +624,12 @@ static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool &x_ok, cudaStream_t 
         return COLA_SUCCESS;
     const int64_t nvec = (a.K + E - 1) / E;
     const size_t bytes = (size_t)g->NX * nvec * 16;
-    if (g->x_pad_bytes < bytes) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        COLA_CUDA(cudaStreamIsCapturing(st, &cap));
-        if (cap != cudaStreamCaptureStatusNone)
-            return COLA_SUCCESS;
-        if (ensure(g->x_pad, g->x_pad_bytes, bytes) != COLA_SUCCESS) {
-            cudaGetLastError();
-            clear_error();
-            return COLA_SUCCESS;
-        }
+    if (capturing && g->x_pad.bytes < bytes)
+        return COLA_SUCCESS;
+    if (grow(g->x_pad, bytes, capturing, g->kept) != COLA_SUCCESS) {
+        cudaGetLastError();
+        clear_error();
+        return COLA_SUCCESS;
     }
     const int64_t total = g->NX * nvec;
     const unsigned blocks = (unsigned)std::min<int64_t>((total + dev::kThreads - 1) / dev::kThreads,
@@ -641,13 +637,13 @@ static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool &x_ok, cudaStream_t 
     t_launches++;
     if (a.xdt == COLA_FLOAT32)
         dev::pad_rows_kernel<float><<<blocks, dev::kThreads, 0, st>>>(
-            static_cast<const float *>(a.X), a.ldx, static_cast<float *>(g->x_pad), (int)nvec, total, a.K);
+            static_cast<const float *>(a.X), a.ldx, g->x_pad.f(), (int)nvec, total, a.K);
     else
         dev::pad_rows_kernel<__nv_bfloat16><<<blocks, dev::kThreads, 0, st>>>(
-            static_cast<const __nv_bfloat16 *>(a.X), a.ldx, static_cast<__nv_bfloat16 *>(g->x_pad), (int)nvec, total,
+            static_cast<const __nv_bfloat16 *>(a.X), a.ldx, static_cast<__nv_bfloat16 *>(g->x_pad.p), (int)nvec, total,
             a.K);
     COLA_CUDA(cudaGetLastError());
-    a.X = g->x_pad;
+    a.X = g->x_pad.p;
     a.ldx = nvec * E;
     x_ok = true;
     return COLA_SUCCESS;
@@ -853,6 +849,35 @@ cola_status ensure(void *&p, size_t &have, size_t need)
     return COLA_SUCCESS;
 }
 
+bool is_capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
+        cudaGetLastError();
+        return true;  // the legacy stream beside a blocking stream's capture
+    }
+    return s != cudaStreamCaptureStatusNone;
+}
+
+cola_status grow(Workspace &w, size_t need, bool capturing, KeptBlocks &kept)
+{
+    if (w.bytes < need) {
+        if (w.captured || capturing) {  // while capturing nothing can be waited for either
+            try {
+                if (w.p)
+                    kept.blocks.push_back({w.p, w.bytes});
+            } catch (const std::bad_alloc &) {
+                return fail(COLA_ERROR_OUT_OF_MEMORY, "workspace: host allocation failed");
+            }
+            w = Workspace();
+        }
+        w.captured = false;
+        COLA_TRY(ensure(w.p, w.bytes, need));
+    }
+    w.captured = w.captured || capturing;
+    return COLA_SUCCESS;
+}
+
 RowViewParams row_view_params(int64_t nnz, const cola_upload_opts *opts)
 {
     const int64_t warps = (int64_t)sm_count() * 32;
@@ -876,11 +901,10 @@ void graph_release(cola_graph *g)
     cudaGetDevice(&cur);
     cudaSetDevice(g->device);
     device_free(g->dmem);
-    device_free(g->ppl_buf);
-    device_free(g->stage_buf);
-    device_free(g->ws);
-    device_free(g->ws_hub);
-    device_free(g->x_pad);
+    for (void *p : {g->ppl_buf.p, g->stage_buf.p, g->ws.p, g->ws_hub.p, g->x_pad.p})
+        device_free(p);
+    for (const auto &b : g->kept.blocks)
+        device_free(b.first);
     host_pipe_release(g->host_pipe);
     cudaSetDevice(cur);
     delete g;
@@ -1231,8 +1255,8 @@ cola_status cola_graph_get_info(const cola_graph *g, cola_graph_info *o)
     o->local_chunks = g->lchunks;
     o->remote_chunks = g->rchunks;
     o->remote_cols = g->rcols;
-    o->device_bytes = (int64_t)(g->dbytes + g->ppl_bytes + g->stage_bytes + g->ws_bytes + g->ws_hub_bytes +
-                                  g->x_pad_bytes);
+    o->device_bytes = (int64_t)(g->dbytes + g->ppl_buf.bytes + g->stage_buf.bytes + g->ws.bytes + g->ws_hub.bytes +
+                                  g->x_pad.bytes + g->kept.bytes());
     o->hub_rows = g->nhub;
     o->hub_segments = g->nseg;
     o->row_tasks = g->ntask;
@@ -1324,14 +1348,14 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
     cudaStream_t st = (cudaStream_t)stream;
     if (g->N == 0)
         return COLA_SUCCESS;
+    const bool capturing = is_capturing(st);
 
     if (schedule == COLA_SCHEDULE_ROWS) {
         // one writer per output row: Y written directly in its own dtype
         // rows of the hub workspace are whole vectors of X
         const int64_t E = xdt == COLA_FLOAT32 ? 4 : 8, ldw = (K + E - 1) / E * E;
         if (g->nseg > 0)
-            COLA_TRY(ensure(reinterpret_cast<void *&>(g->ws_hub), g->ws_hub_bytes,
-                            (size_t)g->nseg * ldw * sizeof(float)));
+            COLA_TRY(grow(g->ws_hub, (size_t)g->nseg * ldw * sizeof(float), capturing, g->kept));
         RowsLaunch a;
         a.ra.rowptr = g->rv_ptr;
         a.ra.col = g->rv_col;
@@ -1342,7 +1366,7 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         a.ra.seg_beg = g->seg_beg;
         a.ra.nseg = g->nseg;
         a.ra.seg_len = g->hub_segment;
-        a.ra.ws = g->ws_hub;
+        a.ra.ws = g->ws_hub.f();
         a.ra.ld_ws = ldw;
         a.X = X;
         a.ldx = ldx;
@@ -1358,11 +1382,11 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         a.k_tile = opts ? opts->k_tile : 0;
         bool x_ok = a.vec;
         if (!a.vec)
-            COLA_TRY(pad_x(g, a, x_ok, st));
+            COLA_TRY(pad_x(g, a, x_ok, capturing, st));
         if (a.vec)
-            COLA_TRY(launch_block(block_args(g, g->ws_hub, ldw), a, st));
+            COLA_TRY(launch_block(block_args(g, g->ws_hub.f(), ldw), a, st));
         else if (x_ok)
-            COLA_TRY(launch_block_odd(block_args(g, g->ws_hub, ldw), a, st));
+            COLA_TRY(launch_block_odd(block_args(g, g->ws_hub.f(), ldw), a, st));
         else
             COLA_TRY(launch_rows(a, st));
         if (g->nhub > 0 && x_ok) {
@@ -1371,11 +1395,11 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
             using BF = __nv_bfloat16;
             if (ydt == COLA_FLOAT32) {
                 auto fn = a.vec ? dev::hub_combine_vec_kernel<float, true> : dev::hub_combine_vec_kernel<float, false>;
-                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw,
+                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw,
                                         static_cast<float *>(Y), ldy, K, accumulate));
             } else {
                 auto fn = a.vec ? dev::hub_combine_vec_kernel<BF, true> : dev::hub_combine_vec_kernel<BF, false>;
-                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw,
+                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw,
                                         static_cast<BF *>(Y), ldy, K, accumulate));
             }
         } else if (g->nhub > 0) {
@@ -1383,10 +1407,10 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
             t_launches++;
             if (ydt == COLA_FLOAT32)
                 dev::hub_combine_kernel<float><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw, static_cast<float *>(Y), ldy, K, accumulate);
+                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw, static_cast<float *>(Y), ldy, K, accumulate);
             else
                 dev::hub_combine_kernel<__nv_bfloat16><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub, ldw, static_cast<__nv_bfloat16 *>(Y), ldy, K,
+                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw, static_cast<__nv_bfloat16 *>(Y), ldy, K,
                     accumulate);
             COLA_CUDA(cudaGetLastError());
         }
@@ -1400,8 +1424,8 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         acc = static_cast<float *>(Y);
         ldacc = ldy;
     } else {
-        COLA_TRY(ensure(reinterpret_cast<void *&>(g->ws), g->ws_bytes, (size_t)g->N * K * sizeof(float)));
-        acc = g->ws;
+        COLA_TRY(grow(g->ws, (size_t)g->N * K * sizeof(float), capturing, g->kept));
+        acc = g->ws.f();
         ldacc = K;
     }
     if (!accumulate) {
@@ -1422,7 +1446,7 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         // local chunks of every partition, then per partition the remote rows in
         // batches: gather into the HBM staging buffer, scatter from it.
         const int64_t ldst = (K + 7) / 8 * 8;
-        COLA_TRY(ensure(g->stage_buf, g->stage_bytes, (size_t)2 * batch_rows * ldst * esz));
+        COLA_TRY(grow(g->stage_buf, (size_t)2 * batch_rows * ldst * esz, capturing, g->kept));
         // one launch for the local parts: r_num = 0 via a host copy of the table
         {
             FusedArgs a{nullptr, part_desc_zero(), 1, 0, X, ldx, acc, ldacc, K, xdt,
@@ -1441,7 +1465,7 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
             const PartDesc &full = g->h_fused[(size_t)p];
             for (int32_t b0 = 0; b0 < full.r_num; b0 += batch_rows) {
                 const int32_t nb = std::min(batch_rows, full.r_num - b0);
-                char *sb = static_cast<char *>(g->stage_buf) + (size_t)(pp & 1) * batch_rows * ldst * esz;
+                char *sb = static_cast<char *>(g->stage_buf.p) + (size_t)(pp & 1) * batch_rows * ldst * esz;
                 pp++;
                 GatherSeg s;
                 std::memset(&s, 0, sizeof s);
@@ -1464,7 +1488,7 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
     } else {  // PIPELINE
         const int64_t ld = ldx;
         const size_t per_pe = (size_t)g->npp * ld * esz;
-        COLA_TRY(ensure(g->ppl_buf, g->ppl_bytes, 2 * (size_t)P * per_pe));
+        COLA_TRY(grow(g->ppl_buf, 2 * (size_t)P * per_pe, capturing, g->kept));
         // stage 0: local + intra-group remote of every PE (.cuh:797-805)
         {
             FusedArgs a{g->d_stage0, part_desc_zero(), P, g->stage0_total, X, ldx, acc, ldacc, K, xdt,
@@ -1472,7 +1496,7 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
             COLA_TRY(launch_fused(a, st));
         }
         for (int32_t s = 1; s < g->nstages; s++) {
-            char *buf = static_cast<char *>(g->ppl_buf) + (size_t)((s - 1) % 2) * P * per_pe;
+            char *buf = static_cast<char *>(g->ppl_buf.p) + (size_t)((s - 1) % 2) * P * per_pe;
             // every PE's put for stage s (batching_data_ppl + put_nbi, .cuh:788-793/811-816)
             COLA_TRY(launch_gather(g->d_put[(size_t)s - 1], GatherSeg{}, P, g->put_total[(size_t)s - 1], X, ldx,
                                    buf, ld, K, xdt, st));
