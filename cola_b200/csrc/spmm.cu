@@ -346,75 +346,19 @@ static cola_status launch_gather(const GatherSeg *segs, const GatherSeg &single,
 // row-major schedule dispatch
 // ---------------------------------------------------------------------------
 struct RowsLaunch {
-    dev::RowsArgs ra;
     const void *X;
     int64_t ldx;
     void *Y;
     int64_t ldy;
     int K;
     cola_dtype xdt, ydt;
-    bool vec;
+    bool vec;   // rows of X and Y are read and written in vectors
+    bool xvec;  // those of X
     int accumulate;
     int unroll;
     int min_blocks;
     int k_tile;
 };
-
-template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC>
-static cola_status launch_rows_t(const RowsLaunch &a, cudaStream_t st)
-{
-    using T = typename dev::ElemOf<TR>::T;
-    constexpr int W = LG * NV * TR::E;
-    auto fn = dev::rows_spmm_kernel<TR, TY, LG, NV, UNROLL, VEC>;
-    const int64_t gx = grid_for((const void *)fn, a.ra.nseg + a.ra.nrows);
-    const int gy = (a.K + W - 1) / W;
-    t_launches++;
-    fn<<<dim3((unsigned)gx, (unsigned)gy), dev::kThreads, 0, st>>>(a.ra, static_cast<const T *>(a.X), a.ldx,
-                                                                   static_cast<TY *>(a.Y), a.ldy, a.K, a.accumulate);
-    COLA_CUDA(cudaGetLastError());
-    return COLA_SUCCESS;
-}
-
-template <typename TR, typename TY, bool VEC>
-static cola_status launch_rows_geo(const RowsLaunch &a, int V, cudaStream_t st)
-{
-    if (V <= 1)
-        return launch_rows_t<TR, TY, 1, 1, 4, VEC>(a, st);
-    if (V <= 2)
-        return launch_rows_t<TR, TY, 2, 1, 4, VEC>(a, st);
-    if (V <= 4)
-        return launch_rows_t<TR, TY, 4, 1, 4, VEC>(a, st);
-    if (V <= 8)
-        return launch_rows_t<TR, TY, 8, 1, 4, VEC>(a, st);
-    if (V <= 16)
-        return launch_rows_t<TR, TY, 16, 1, 4, VEC>(a, st);
-    if (V <= 32) {
-        if (a.unroll == 8)
-            return launch_rows_t<TR, TY, 32, 1, 8, VEC>(a, st);
-        if (a.unroll == 2)
-            return launch_rows_t<TR, TY, 32, 1, 2, VEC>(a, st);
-        return launch_rows_t<TR, TY, 32, 1, 4, VEC>(a, st);
-    }
-    if (V <= 64) {
-        if (a.unroll == 4 || a.unroll == 8)
-            return launch_rows_t<TR, TY, 32, 2, 4, VEC>(a, st);
-        return launch_rows_t<TR, TY, 32, 2, 2, VEC>(a, st);
-    }
-    return launch_rows_t<TR, TY, 32, 4, 2, VEC>(a, st);
-}
-
-// Element by element (pad_x says when).
-static cola_status launch_rows(const RowsLaunch &a, cudaStream_t st)
-{
-    if (a.ra.nseg + a.ra.nrows <= 0 || a.K <= 0)
-        return COLA_SUCCESS;
-    using BF = __nv_bfloat16;
-    if (a.xdt == COLA_FLOAT32)
-        return a.ydt == COLA_FLOAT32 ? launch_rows_geo<dev::ScalarTraits<float>, float, false>(a, a.K, st)
-                                     : launch_rows_geo<dev::ScalarTraits<float>, BF, false>(a, a.K, st);
-    return a.ydt == COLA_FLOAT32 ? launch_rows_geo<dev::ScalarTraits<BF>, float, false>(a, a.K, st)
-                                 : launch_rows_geo<dev::ScalarTraits<BF>, BF, false>(a, a.K, st);
-}
 
 template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB = 1>
 static cola_status launch_block_t(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
@@ -443,7 +387,8 @@ static cola_status launch_block_t(const dev::BlockArgs &ba, const RowsLaunch &a,
     return COLA_SUCCESS;
 }
 
-// Element-wise output (VEC_Y false): the default geometry of the width.
+// Element-wise output (VEC_Y false), X in vectors or element by element: the
+// default geometry of the width.
 template <typename TR, typename TY, int LG, int NV, int UNROLL, int MINB>
 static cola_status launch_block_odd_t(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
 {
@@ -463,31 +408,39 @@ template <typename TR, typename TY>
 static cola_status launch_block_odd_geo(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
 {
     const int V = (a.K + TR::E - 1) / TR::E;
+    // eight values of BF16 one by one: 64 registers a thread would spill
+    constexpr bool wide = dev::kLoose<TR> && TR::E == 8;
+    constexpr int M = wide ? 2 : 4, M2 = wide ? 2 : 3;
     if (V <= 1)
-        return launch_block_odd_t<TR, TY, 1, 1, 1, 4>(ba, a, st);
+        return launch_block_odd_t<TR, TY, 1, 1, 1, M>(ba, a, st);
     if (V <= 2)
-        return launch_block_odd_t<TR, TY, 2, 1, 2, 4>(ba, a, st);
+        return launch_block_odd_t<TR, TY, 2, 1, 2, M>(ba, a, st);
     if (V <= 4)
-        return launch_block_odd_t<TR, TY, 4, 1, 4, 4>(ba, a, st);
+        return launch_block_odd_t<TR, TY, 4, 1, 4, M>(ba, a, st);
     if (V <= 8)
-        return launch_block_odd_t<TR, TY, 8, 1, 4, 4>(ba, a, st);
+        return launch_block_odd_t<TR, TY, 8, 1, 4, M>(ba, a, st);
     if (V <= 16)
-        return launch_block_odd_t<TR, TY, 16, 1, 4, 4>(ba, a, st);
+        return launch_block_odd_t<TR, TY, 16, 1, 4, M>(ba, a, st);
     if (V <= 32)
-        return launch_block_odd_t<TR, TY, 32, 1, 4, 4>(ba, a, st);
-    return launch_block_odd_t<TR, TY, 32, 2, 4, 3>(ba, a, st);
+        return launch_block_odd_t<TR, TY, 32, 1, 4, M>(ba, a, st);
+    return launch_block_odd_t<TR, TY, 32, 2, 4, M2>(ba, a, st);
+}
+
+template <typename T>
+static cola_status launch_block_odd_x(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
+{
+    if (a.ydt == COLA_FLOAT32)
+        return a.xvec ? launch_block_odd_geo<dev::VecTraits<T>, float>(ba, a, st)
+                      : launch_block_odd_geo<dev::LooseTraits<T>, float>(ba, a, st);
+    return a.xvec ? launch_block_odd_geo<dev::VecTraits<T>, __nv_bfloat16>(ba, a, st)
+                  : launch_block_odd_geo<dev::LooseTraits<T>, __nv_bfloat16>(ba, a, st);
 }
 
 static cola_status launch_block_odd(const dev::BlockArgs &ba, const RowsLaunch &a, cudaStream_t st)
 {
     if (ba.nitem <= 0)
         return COLA_SUCCESS;
-    using BF = __nv_bfloat16;
-    if (a.xdt == COLA_FLOAT32)
-        return a.ydt == COLA_FLOAT32 ? launch_block_odd_geo<dev::VecTraits<float>, float>(ba, a, st)
-                                     : launch_block_odd_geo<dev::VecTraits<float>, BF>(ba, a, st);
-    return a.ydt == COLA_FLOAT32 ? launch_block_odd_geo<dev::VecTraits<BF>, float>(ba, a, st)
-                                 : launch_block_odd_geo<dev::VecTraits<BF>, BF>(ba, a, st);
+    return a.xdt == COLA_FLOAT32 ? launch_block_odd_x<float>(ba, a, st) : launch_block_odd_x<__nv_bfloat16>(ba, a, st);
 }
 
 // Narrow passes (a full warp on a 64- or 128-feature tile, 8 or 4 bytes per
@@ -608,24 +561,22 @@ bool vec_ok_rows(cola_dtype xdt, const void *X, int64_t ldx, cola_dtype ydt, con
     return true;
 }
 
-// X as the vector form reads it: itself where its rows are whole aligned
-// vectors, else a padded copy in the graph's workspace (x_ok false: neither).
-// The copy is two passes over X against one over X per entry of a row, so it is
-// made from 2 entries a row on; not while the stream is being captured with too
-// small a workspace (allocating would break the capture), nor when the device
-// has no room for it.  The scalar kernel remains for those calls.  K = 33 FP32,
-// 150 K rows, 2.4 M entries: 185 -> 73 us, K = 74 BF16 209 -> 100, K = 301 FP32
-// 717 -> 337, K = 33 at 3 entries a row 86 -> 42.
-static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool &x_ok, bool capturing, cudaStream_t st)
+// X as the vector form reads it (a.xvec): itself where its rows are whole
+// aligned vectors, else a padded copy in the graph's workspace, else (few entries
+// a row, or no room on the device) left for the element-wise form, which gives
+// the same bits.  The copy is two passes over X, the element-wise form issues E
+// loads for one vector: padded from 16 entries a row on for FP32 X and 4 for BF16
+// (200 K rows, uniform, padded against element-wise in us: K = 33 FP32 at 4, 16,
+// 24 entries a row 54 / 44, 91 / 90, 113 / 118; K = 301 FP32 at 16 and 48 640 /
+// 606, 1460 / 1637; K = 33 BF16 at 2, 4, 16 39 / 34, 46 / 46, 77 / 104).
+static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool capturing, cudaStream_t st)
 {
     const int E = a.xdt == COLA_FLOAT32 ? 4 : 8, esz = 16 / E;
-    x_ok = a.K % E == 0 && a.ldx % E == 0 && a.ldx <= INT32_MAX / esz && aligned16(a.X);
-    if (x_ok || g->nnz_l + g->nnz_r < 2 * (int64_t)g->NX)
+    a.xvec = a.K % E == 0 && a.ldx % E == 0 && a.ldx <= INT32_MAX / esz && aligned16(a.X);
+    if (a.xvec || g->nnz_l + g->nnz_r < (E == 4 ? 16 : 4) * (int64_t)g->NX)
         return COLA_SUCCESS;
     const int64_t nvec = (a.K + E - 1) / E;
     const size_t bytes = (size_t)g->NX * nvec * 16;
-    if (capturing && g->x_pad.bytes < bytes)
-        return COLA_SUCCESS;
     if (grow(g->x_pad, bytes, capturing, g->kept) != COLA_SUCCESS) {
         cudaGetLastError();
         clear_error();
@@ -645,7 +596,7 @@ static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool &x_ok, bool capturin
     COLA_CUDA(cudaGetLastError());
     a.X = g->x_pad.p;
     a.ldx = nvec * E;
-    x_ok = true;
+    a.xvec = true;
     return COLA_SUCCESS;
 }
 
@@ -1357,17 +1308,6 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         if (g->nseg > 0)
             COLA_TRY(grow(g->ws_hub, (size_t)g->nseg * ldw * sizeof(float), capturing, g->kept));
         RowsLaunch a;
-        a.ra.rowptr = g->rv_ptr;
-        a.ra.col = g->rv_col;
-        a.ra.val = g->rv_val;
-        a.ra.nrows = g->N;
-        a.ra.hub_threshold = g->hub_threshold;
-        a.ra.seg_row = g->seg_row;
-        a.ra.seg_beg = g->seg_beg;
-        a.ra.nseg = g->nseg;
-        a.ra.seg_len = g->hub_segment;
-        a.ra.ws = g->ws_hub.f();
-        a.ra.ld_ws = ldw;
         a.X = X;
         a.ldx = ldx;
         a.Y = Y;
@@ -1380,16 +1320,12 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
         a.unroll = opts ? opts->unroll : 0;
         a.min_blocks = opts ? opts->min_blocks : 0;
         a.k_tile = opts ? opts->k_tile : 0;
-        bool x_ok = a.vec;
+        a.xvec = a.vec;
         if (!a.vec)
-            COLA_TRY(pad_x(g, a, x_ok, capturing, st));
-        if (a.vec)
-            COLA_TRY(launch_block(block_args(g, g->ws_hub.f(), ldw), a, st));
-        else if (x_ok)
-            COLA_TRY(launch_block_odd(block_args(g, g->ws_hub.f(), ldw), a, st));
-        else
-            COLA_TRY(launch_rows(a, st));
-        if (g->nhub > 0 && x_ok) {
+            COLA_TRY(pad_x(g, a, capturing, st));
+        const dev::BlockArgs ba = block_args(g, g->ws_hub.f(), ldw);
+        COLA_TRY(a.vec ? launch_block(ba, a, st) : launch_block_odd(ba, a, st));
+        if (g->nhub > 0) {
             const unsigned blocks = hub_blocks(g->nhub * dev::hub_tiles(K), dev::hub_lanes(K));
             t_launches++;
             using BF = __nv_bfloat16;
@@ -1402,17 +1338,6 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
                 COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw,
                                         static_cast<BF *>(Y), ldy, K, accumulate));
             }
-        } else if (g->nhub > 0) {
-            const int64_t blocks = (g->nhub + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock;
-            t_launches++;
-            if (ydt == COLA_FLOAT32)
-                dev::hub_combine_kernel<float><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw, static_cast<float *>(Y), ldy, K, accumulate);
-            else
-                dev::hub_combine_kernel<__nv_bfloat16><<<(unsigned)blocks, dev::kThreads, 0, st>>>(
-                    g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw, static_cast<__nv_bfloat16 *>(Y), ldy, K,
-                    accumulate);
-            COLA_CUDA(cudaGetLastError());
         }
         return COLA_SUCCESS;
     }

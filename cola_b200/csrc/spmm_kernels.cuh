@@ -164,8 +164,43 @@ struct ScalarTraits {
     __device__ __forceinline__ static void unpack(const raw_t &r, float (&f)[1]) { f[0] = (float)r; }
 };
 
+// Rows of X read element by element (their start is not 16-byte aligned, or K
+// ends inside a vector): as many features a lane as VecTraits, but LG apart, so
+// that neighbouring lanes read neighbouring elements.  A feature is summed by
+// the same lane group in the same order as in the vector form: the same bits.
+template <typename T>
+struct LooseTraits {
+    static constexpr int E = 16 / (int)sizeof(T);
+    struct raw_t {
+        T v[E];
+    };
+    // Elements p[q * step] for q * step < left.
+    __device__ __forceinline__ static raw_t load(const T *p, int step, int left)
+    {
+        raw_t r;
+#pragma unroll
+        for (int q = 0; q < E; q++)
+            r.v[q] = q * step < left ? __ldg(p + q * step) : T(0.f);
+        return r;
+    }
+    __device__ __forceinline__ static void unpack(const raw_t &r, float (&f)[E])
+    {
+#pragma unroll
+        for (int q = 0; q < E; q++)
+            f[q] = (float)r.v[q];
+    }
+};
+template <typename TR>
+constexpr bool kLoose = false;
+template <typename T>
+constexpr bool kLoose<LooseTraits<T>> = true;
+
 template <typename TR>
 struct ElemOf;
+template <typename U>
+struct ElemOf<LooseTraits<U>> {
+    using T = U;
+};
 template <>
 struct ElemOf<VecTraits<float>> {
     using T = float;

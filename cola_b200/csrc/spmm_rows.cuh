@@ -93,145 +93,17 @@ __device__ __forceinline__ void store_out<__nv_bfloat16, 1, false>(__nv_bfloat16
     *p = __float2bfloat16_rn(a[0]);
 }
 
-// The first `left` (at most E) of a lane's values, one element at a time: an
-// output whose rows are not vector-aligned or end inside a vector.
-template <typename TY, int E>
+// A lane's values one element at a time, STEP apart, as far as `left`: an output
+// whose rows are not vector-aligned or end inside a vector.
+template <typename TY, int E, int STEP = 1>
 __device__ __forceinline__ void store_some(TY *p, const float (&a)[E], bool accumulate, int left)
 {
 #pragma unroll
     for (int q = 0; q < E; q++)
-        if (q < left) {
+        if (q * STEP < left) {
             const float v[1] = {a[q]};
-            store_out<TY, 1, false>(p + q, v, accumulate);
+            store_out<TY, 1, false>(p + q * STEP, v, accumulate);
         }
-}
-
-// Hub segment table: segment s covers entries [beg[s], min(beg[s]+seg_len,
-// rowptr[row[s]+1])) and writes its partial to ws row s.
-struct RowsArgs {
-    const int64_t *rowptr;  // N+1
-    const int32_t *col;     // global column ids (kRowEnd on a row's last entry)
-    const float *val;
-    int32_t nrows;
-    int32_t hub_threshold;  // rows with more entries are handled by segments
-    const int32_t *seg_row;
-    const int64_t *seg_beg;
-    int64_t nseg;
-    int32_t seg_len;
-    float *ws;              // nseg x K FP32 partials
-    int64_t ld_ws;
-};
-
-template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC_Y>
-__global__ void __launch_bounds__(kThreads) rows_spmm_kernel(const __grid_constant__ RowsArgs ra,
-                                                             const typename ElemOf<TR>::T *__restrict__ X,
-                                                             int64_t ldx, TY *__restrict__ Y, int64_t ldy, int K,
-                                                             int accumulate)
-{
-    using T = typename ElemOf<TR>::T;
-    using raw_t = typename TR::raw_t;
-    constexpr int E = TR::E;
-    constexpr int G = 32 / LG;
-    constexpr int W = LG * NV * E;
-    const int lane = threadIdx.x & 31;
-    const int g = lane / LG;
-    const int gl = lane % LG;
-    const int k0 = blockIdx.y * W;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    const int64_t total = ra.nseg + ra.nrows;
-    bool kok[NV];
-#pragma unroll
-    for (int j = 0; j < NV; j++)
-        kok[j] = (k0 + (gl + j * LG) * E) < K;
-    const T *xk = X + k0;
-
-    for (int64_t it = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); it < total; it += nwarps) {
-        int64_t b, e;
-        bool to_ws;
-        int64_t out_row;
-        if (it < ra.nseg) {
-            const int32_t r = __ldg(ra.seg_row + it);
-            b = __ldg(ra.seg_beg + it);
-            e = min(b + (int64_t)ra.seg_len, __ldg(ra.rowptr + r + 1));
-            to_ws = true;
-            out_row = it;
-        } else {
-            const int64_t r = it - ra.nseg;
-            b = __ldg(ra.rowptr + r);
-            e = __ldg(ra.rowptr + r + 1);
-            if (e - b > ra.hub_threshold)
-                continue;  // written by the hub combine
-            to_ws = false;
-            out_row = r;
-        }
-        float acc[NV][E];
-#pragma unroll
-        for (int j = 0; j < NV; j++)
-#pragma unroll
-            for (int q = 0; q < E; q++)
-                acc[j][q] = 0.f;
-        for (int64_t base = b; base < e; base += 32) {
-            const int n = (int)min((int64_t)32, e - base);
-            int mc = 0;
-            float mv = 0.f;
-            if (lane < n) {
-                mc = __ldg(ra.col + base + lane) & kColMask;
-                mv = __ldg(ra.val + base + lane);
-            }
-            for (int jj = 0; jj < n; jj += G * UNROLL) {
-                raw_t xr[UNROLL][NV];
-                float vv[UNROLL];
-#pragma unroll
-                for (int u = 0; u < UNROLL; u++) {
-                    const int k = jj + u * G + g;
-                    const int cc = __shfl_sync(kFull, mc, k & 31);
-                    const float v = __shfl_sync(kFull, mv, k & 31);
-                    const bool ok = k < n;
-                    vv[u] = ok ? v : 0.f;
-                    const T *xp = xk + (int64_t)cc * ldx;
-#pragma unroll
-                    for (int j = 0; j < NV; j++)
-                        xr[u][j] = (ok && kok[j]) ? TR::load(xp + (gl + j * LG) * E) : TR::zero();
-                }
-#pragma unroll
-                for (int u = 0; u < UNROLL; u++)
-#pragma unroll
-                    for (int j = 0; j < NV; j++) {
-                        float f[E];
-                        TR::unpack(xr[u][j], f);
-#pragma unroll
-                        for (int q = 0; q < E; q++)
-                            acc[j][q] = fmaf(vv[u], f[q], acc[j][q]);
-                    }
-            }
-        }
-#pragma unroll
-        for (int off = LG; off < 32; off <<= 1)
-#pragma unroll
-            for (int j = 0; j < NV; j++)
-#pragma unroll
-                for (int q = 0; q < E; q++)
-                    acc[j][q] += __shfl_xor_sync(kFull, acc[j][q], off);
-        if (g == 0) {
-            if (to_ws) {
-                float *wp = ra.ws + out_row * ra.ld_ws + k0;
-#pragma unroll
-                for (int j = 0; j < NV; j++)
-                    if (kok[j]) {
-                        float *p = wp + (gl + j * LG) * E;
-#pragma unroll
-                        for (int q = 0; q < E; q++)
-                            p[q] = acc[j][q];
-                    }
-            } else {
-                TY *yp = Y + out_row * ldy + k0;
-#pragma unroll
-                for (int j = 0; j < NV; j++)
-                    if (kok[j])
-                        store_out<TY, E, VEC_Y>(yp + (gl + j * LG) * E, acc[j], accumulate != 0);
-            }
-        }
-    }
 }
 
 // Work items of the streaming form, segments first, then tasks, one 16-byte
@@ -349,11 +221,15 @@ struct RowStream {
     static constexpr int G = 32 / LG;
     static constexpr int R = G * UNROLL;  // entries per round
     static constexpr int LANES = LG, NVEC = NV;
+    static constexpr bool LOOSE = kLoose<TR>;
+    static constexpr int STEP = LOOSE ? LG : 1;  // between a lane's features of one vector
+    static_assert(!LOOSE || (!VEC_Y && !RED), "element-wise X goes with element-wise Y");
     static_assert(32 % R == 0 && (NV == 1 || LG == 32), "rounds must divide the 32-entry batch");
 
     float2 acc[NV][E / 2];
     const char *xk;  // X + the lane's first feature
     int32_t ldxb;    // bytes between rows (the vector path's fit 31 bits)
+    int64_t ldxe;    // elements between rows (LOOSE)
     TY *Y;
     int64_t ldy;
     int koff;  // the lane's first feature
@@ -370,8 +246,9 @@ struct RowStream {
         g = lane / LG;
         gl = lane % LG;
         ldxb = (int32_t)(ldx_ * (int64_t)sizeof(T));
+        ldxe = ldx_;
         ldy = ldy_;
-        koff = k0 + gl * E;
+        koff = k0 + gl * (LOOSE ? 1 : E);
         xk = reinterpret_cast<const char *>(X + koff);
         Y = Y_;
         accumulate = acc_ != 0;
@@ -395,6 +272,8 @@ struct RowStream {
     {
         if constexpr (RED)
             red_add<N, true>(p, a);
+        else if constexpr (LOOSE)
+            store_some<TO, N, STEP>(p, a, add, left);
         else if constexpr (VEC_Y)
             store_out<TO, N, (N > 1)>(p, a, add);
         else if (to_ws)
@@ -453,7 +332,7 @@ struct RowStream {
 #pragma unroll
                 for (int q = 0; q < EO; q++)
                     a[q] = v[q];
-                put(p + f, a, add, K - koff - f);
+                put(p + f * STEP, a, add, K - koff - f * STEP);
             }
         }
         clear();
@@ -480,11 +359,18 @@ struct RowStream {
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) {
             if (ALL || u * G + g < cnt) {
-                const T *xp = reinterpret_cast<const T *>(row_at(xk, c[u], ldxb));
+                if constexpr (LOOSE) {
+                    const T *xp = reinterpret_cast<const T *>(xk) + (int64_t)c[u] * ldxe;
 #pragma unroll
-                for (int j = 0; j < NV; j++)
-                    if (kok[j])
-                        xr[u][j] = TR::load(xp + j * LG * E);
+                    for (int j = 0; j < NV; j++)
+                        xr[u][j] = TR::load(xp + j * LG * E, LG, K - koff - j * LG * E);
+                } else {
+                    const T *xp = reinterpret_cast<const T *>(row_at(xk, c[u], ldxb));
+#pragma unroll
+                    for (int j = 0; j < NV; j++)
+                        if (kok[j])
+                            xr[u][j] = TR::load(xp + j * LG * E);
+                }
             }
         }
     }
@@ -769,42 +655,10 @@ __global__ void __launch_bounds__(kThreads, MINB) rowblock_tiled_kernel(const __
     }
 }
 
-// Hub rows: sum the segment partials ws[s0 .. s1) pairwise — a binary tree in
-// fixed order, computed in place in the workspace by the owning lane — and
-// write the row.  One warp per hub row; lane l owns features l, l+32, ...
-template <typename TY>
-__global__ void __launch_bounds__(kThreads) hub_combine_kernel(const int32_t *__restrict__ hub_row,
-                                                              const int64_t *__restrict__ hub_seg, int64_t nhub,
-                                                              float *__restrict__ ws, int64_t ld_ws, TY *__restrict__ Y,
-                                                              int64_t ldy, int K, int accumulate)
-{
-    const int lane = threadIdx.x & 31;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    for (int64_t h = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); h < nhub; h += nwarps) {
-        const int64_t s0 = hub_seg[h], m = hub_seg[h + 1] - s0;
-        float *w0 = ws + s0 * ld_ws;
-        for (int64_t stride = 1; stride < m; stride <<= 1)
-            for (int64_t i = 0; i + stride < m; i += 2 * stride) {
-                float *a = w0 + i * ld_ws;
-                const float *c = w0 + (i + stride) * ld_ws;
-                for (int k = lane; k < K; k += 32)
-                    a[k] += c[k];
-            }
-        TY *yp = Y + (int64_t)hub_row[h] * ldy;
-        for (int k = lane; k < K; k += 32) {
-            const float v = w0[k];
-            if constexpr (sizeof(TY) == 4)
-                yp[k] = accumulate ? (float)yp[k] + v : v;
-            else
-                yp[k] = __float2bfloat16_rn(v);
-        }
-    }
-}
-
-// Hub rows, 16-byte vector form (ws rows 16-byte aligned, of whole vectors):
-// a group of lc lanes (32, or the power of two that covers K / 4 below) owns one
-// (hub, 4 * lc-feature tile).  The m partials are added pairwise in the order of
-// a binary counter: partial i closes the running block sums of sizes 1, 2, 4,
+// Hub rows (workspace rows are 16-byte aligned and whole vectors): a group of lc
+// lanes (32, or the power of two that covers K / 4 below) owns one (hub, 4 *
+// lc-feature tile).  The m partials are added pairwise in the order of a binary
+// counter: partial i closes the running block sums of sizes 1, 2, 4,
 // ... that its index's trailing one bits name, and the open blocks at the end
 // are folded larger (earlier) first.  The counter is run kHubRadix partials at a
 // time, all their loads in flight and every running sum in a register: whole

@@ -39,7 +39,7 @@ def capture(g, X, Y, schedule):
     (32, 256, 48, S.SCHEDULE_BUFFER, torch.float32)])
 @pytest.mark.parametrize("warm", [True, False])
 def test_replay_after_growth(K, wider, thr, schedule, ydt, warm):
-    n, row, col, val, ps = graph_case(13, 12, seed=5, nparts=2)
+    n, row, col, val, ps = graph_case(13, 32, seed=5, nparts=2)  # dense enough for padded copies of X
     g = S.Graph(ps, hub_threshold=thr)
     X = torch.from_numpy(dense_x(n, K, seed=1)).to(DEV)
     ref = fp64_reference(n, row, col, val, X.cpu().numpy())
