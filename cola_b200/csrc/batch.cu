@@ -33,12 +33,15 @@ struct cola_batch {
     std::vector<BatchGraph> h_desc;  // graphs that run in the batched launch
     BatchGraph *d_desc = nullptr;
     size_t d_desc_bytes = 0;
-    float *d_ws = nullptr;  // hub partials of the batched graphs
+    // hub partials of every graph; for those that run alone work-item counters and
+    // room for the padded copy of X (one after another, so one for all)
+    void *d_ws = nullptr;
     size_t d_ws_bytes = 0;
     cola::BatchLaunch launch = {};  // groups and totals of h_desc
     int64_t total_items = 0, total_hub = 0;
-    struct Solo {  // graphs that run through cola_spmm (scalar path or K > 32 vectors)
+    struct Solo {  // graphs whose operands are not whole vectors: launches of their own
         int g;
+        cola::RowsWork work;
         const void *X;
         int64_t ldx;
         void *Y;
@@ -208,14 +211,11 @@ static cola_status batch_run(cola_batch *b, const cola_spmm_opts *opts, cudaStre
     L.queue = reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(b->d_desc) +
                                                batch_queue_offset(b->h_desc.size() * sizeof(BatchGraph)));
     COLA_TRY(launch_batch(L, st));
-    for (const cola_batch::Solo &s : b->solo) {
-        cola_spmm_opts o;
-        std::memset(&o, 0, sizeof o);
-        o.accumulate = accumulate;
-        o.schedule = COLA_SCHEDULE_ROWS;
-        COLA_TRY(cola_spmm(b->graphs[(size_t)s.g], s.X, b->xdt, s.ldx, s.Y, b->ydt, s.ldy, s.K, &o,
-                           (cola_stream_t)st));
-    }
+    cola_spmm_opts o;
+    std::memset(&o, 0, sizeof o);
+    o.accumulate = accumulate;
+    for (const cola_batch::Solo &s : b->solo)
+        COLA_TRY(rows_product(b->graphs[(size_t)s.g], s.work, s.X, b->xdt, s.ldx, s.Y, b->ydt, s.ldy, s.K, &o, st));
     b->last_launches = t_launches - before;
     return COLA_SUCCESS;
 }
@@ -262,6 +262,92 @@ static std::string tune_key(const cola_batch *b)
     char buf[512];
     std::snprintf(buf, sizeof buf, "%s|%d|%016llx", name.c_str(), prop.multiProcessorCount, (unsigned long long)h);
     return buf;
+}
+
+static cola_status batch_bind(cola_batch *b, const void *const *X, const int64_t *ldx, void *const *Y,
+                              const int64_t *ldy, const int32_t *K, cola_dtype xdt, cola_dtype ydt, cudaStream_t st)
+{
+    COLA_REQUIRE(b && X && ldx && Y && ldy && K, COLA_ERROR_INVALID_ARGUMENT, "cola_batch_bind: null argument");
+    COLA_REQUIRE((xdt == COLA_FLOAT32 || xdt == COLA_BFLOAT16) && (ydt == COLA_FLOAT32 || ydt == COLA_BFLOAT16),
+                 COLA_ERROR_INVALID_ARGUMENT, "cola_batch_bind: unknown dtype");
+    b->bound = false;
+    b->xdt = xdt;
+    b->ydt = ydt;
+    b->h_desc.clear();
+    b->solo.clear();
+    b->total_items = 0;
+    b->total_hub = 0;
+    std::vector<size_t> ws_off;  // of each batched graph's hub partials
+    size_t ws_bytes = 0, pad_bytes = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = ws_bytes;
+        ws_bytes += (bytes + 255) & ~(size_t)255;
+        return at;
+    };
+    constexpr size_t kCounters = (dev::kMaxItemQueues + 1) * sizeof(unsigned int);
+    for (size_t i = 0; i < b->graphs.size(); i++) {
+        cola_graph *g = b->graphs[i];
+        COLA_REQUIRE(K[i] >= 1 && ldx[i] >= K[i] && ldy[i] >= K[i] && (g->N == 0 || (X[i] && Y[i])),
+                     COLA_ERROR_INVALID_ARGUMENT, "cola_batch_bind: graph %zu: K=%d ldx=%lld ldy=%lld", i, K[i],
+                     (long long)ldx[i], (long long)ldy[i]);
+        if (g->N == 0)
+            continue;
+        if (!vec_ok_rows(xdt, X[i], ldx[i], ydt, Y[i], ldy[i], K[i])) {
+            b->solo.push_back({(int)i, {}, X[i], ldx[i], Y[i], ldy[i], K[i]});
+            pad_bytes = std::max(pad_bytes, rows_pad_bytes(g, xdt, X[i], ldx[i], K[i]));
+            continue;
+        }
+        BatchGraph d;
+        // the batch's own hub workspace: offsets here, addresses once it is sized
+        fill_batch_graph(d, g, X[i], ldx[i], Y[i], ldy[i], K[i], xdt, nullptr);
+        ws_off.push_back(place((size_t)g->nseg * K[i] * sizeof(float)));
+        b->total_items += g->nseg + g->ntask;
+        b->h_desc.push_back(d);
+    }
+    const size_t counters = place(b->solo.size() * kCounters);
+    std::vector<size_t> solo_off;
+    for (const cola_batch::Solo &s : b->solo)
+        solo_off.push_back(place((size_t)b->graphs[(size_t)s.g]->nseg * rows_ld_ws(xdt, s.K) * sizeof(float)));
+    const size_t pad = place(0);
+    // without the room for padded rows X is read element by element
+    if (pad_bytes && ensure(b->d_ws, b->d_ws_bytes, ws_bytes + pad_bytes) != COLA_SUCCESS) {
+        cudaGetLastError();
+        clear_error();
+        pad_bytes = 0;
+    }
+    COLA_TRY(ensure(b->d_ws, b->d_ws_bytes, ws_bytes));
+    char *ws = static_cast<char *>(b->d_ws);
+    for (size_t i = 0; i < b->h_desc.size(); i++)
+        b->h_desc[i].ba.ws = reinterpret_cast<float *>(ws + ws_off[i]);
+    for (size_t i = 0; i < b->solo.size(); i++) {
+        cola_batch::Solo &s = b->solo[i];
+        const bool padded = pad_bytes && rows_pad_bytes(b->graphs[(size_t)s.g], xdt, s.X, s.ldx, s.K);
+        s.work = {reinterpret_cast<float *>(ws + solo_off[i]), padded ? ws + pad : nullptr,
+                  reinterpret_cast<unsigned int *>(ws + counters + i * kCounters)};
+    }
+    if (!b->solo.empty())
+        COLA_CUDA(cudaMemsetAsync(ws + counters, 0, b->solo.size() * kCounters, st));
+    COLA_TRY(build_groups(b->h_desc.data(), (int)b->h_desc.size(), b->launch));
+    b->total_hub = b->launch.total_hub;
+    const size_t qoff = batch_queue_offset(b->h_desc.size() * sizeof(BatchGraph));
+    const size_t need = qoff + kBatchQueueBytes;
+    void *p = b->d_desc;
+    COLA_TRY(ensure(p, b->d_desc_bytes, need));
+    b->d_desc = static_cast<BatchGraph *>(p);
+    // the work-item counters start at zero (each launch leaves them so)
+    COLA_CUDA(cudaMemsetAsync(static_cast<char *>(p) + qoff, 0, kBatchQueueBytes, st));
+    if (!b->h_desc.empty())
+        COLA_CUDA(cudaMemcpyAsync(b->d_desc, b->h_desc.data(), b->h_desc.size() * sizeof(BatchGraph),
+                                  cudaMemcpyHostToDevice, st));
+    COLA_CUDA(cudaStreamSynchronize(st));
+    if (b->cexec) {  // a captured graph refers to the old operands
+        cudaGraphExecDestroy(b->cexec);
+        cudaGraphDestroy(b->cgraph);
+        b->cexec = nullptr;
+        b->cgraph = nullptr;
+    }
+    b->bound = true;
+    return COLA_SUCCESS;
 }
 
 }  // namespace cola
@@ -327,65 +413,11 @@ cola_status cola_batch_bind(cola_batch *b, const void *const *X, const int64_t *
                             const int64_t *ldy, const int32_t *K, cola_dtype xdt, cola_dtype ydt,
                             cola_stream_t stream)
 {
-    COLA_REQUIRE(b && X && ldx && Y && ldy && K, COLA_ERROR_INVALID_ARGUMENT, "cola_batch_bind: null argument");
-    COLA_REQUIRE((xdt == COLA_FLOAT32 || xdt == COLA_BFLOAT16) && (ydt == COLA_FLOAT32 || ydt == COLA_BFLOAT16),
-                 COLA_ERROR_INVALID_ARGUMENT, "cola_batch_bind: unknown dtype");
-    cudaStream_t st = (cudaStream_t)stream;
-    b->bound = false;
-    b->xdt = xdt;
-    b->ydt = ydt;
-    b->h_desc.clear();
-    b->solo.clear();
-    b->total_items = 0;
-    b->total_hub = 0;
-    std::vector<size_t> ws_off;  // of each batched graph's hub workspace
-    size_t ws_floats = 0;
-    for (size_t i = 0; i < b->graphs.size(); i++) {
-        cola_graph *g = b->graphs[i];
-        COLA_REQUIRE(K[i] >= 1 && ldx[i] >= K[i] && ldy[i] >= K[i] && (g->N == 0 || (X[i] && Y[i])),
-                     COLA_ERROR_INVALID_ARGUMENT, "cola_batch_bind: graph %zu: K=%d ldx=%lld ldy=%lld", i, K[i],
-                     (long long)ldx[i], (long long)ldy[i]);
-        if (g->N == 0)
-            continue;
-        if (!vec_ok_rows(xdt, X[i], ldx[i], ydt, Y[i], ldy[i], K[i])) {
-            b->solo.push_back({(int)i, X[i], ldx[i], Y[i], ldy[i], K[i]});
-            continue;
-        }
-        BatchGraph d;
-        // the batch's own hub workspace: offsets here, addresses once it is sized
-        fill_batch_graph(d, g, X[i], ldx[i], Y[i], ldy[i], K[i], xdt, nullptr);
-        ws_off.push_back(ws_floats);
-        ws_floats += (size_t)g->nseg * K[i];
-        b->total_items += g->nseg + g->ntask;
-        b->h_desc.push_back(d);
+    try {
+        return batch_bind(b, X, ldx, Y, ldy, K, xdt, ydt, (cudaStream_t)stream);
+    } catch (const std::bad_alloc &) {
+        return fail(COLA_ERROR_OUT_OF_MEMORY, "cola_batch_bind: host allocation failed");
     }
-    void *ws = b->d_ws;
-    const cola_status ws_ok = ensure(ws, b->d_ws_bytes, ws_floats * sizeof(float));
-    b->d_ws = static_cast<float *>(ws);
-    COLA_TRY(ws_ok);
-    for (size_t i = 0; i < b->h_desc.size(); i++)
-        b->h_desc[i].ba.ws = b->d_ws + ws_off[i];
-    COLA_TRY(build_groups(b->h_desc.data(), (int)b->h_desc.size(), b->launch));
-    b->total_hub = b->launch.total_hub;
-    const size_t qoff = batch_queue_offset(b->h_desc.size() * sizeof(BatchGraph));
-    const size_t need = qoff + kBatchQueueBytes;
-    void *p = b->d_desc;
-    COLA_TRY(ensure(p, b->d_desc_bytes, need));
-    b->d_desc = static_cast<BatchGraph *>(p);
-    // the work-item counters start at zero (each launch leaves them so)
-    COLA_CUDA(cudaMemsetAsync(static_cast<char *>(p) + qoff, 0, kBatchQueueBytes, st));
-    if (!b->h_desc.empty())
-        COLA_CUDA(cudaMemcpyAsync(b->d_desc, b->h_desc.data(), b->h_desc.size() * sizeof(BatchGraph),
-                                  cudaMemcpyHostToDevice, st));
-    COLA_CUDA(cudaStreamSynchronize(st));
-    if (b->cexec) {  // a captured graph refers to the old operands
-        cudaGraphExecDestroy(b->cexec);
-        cudaGraphDestroy(b->cgraph);
-        b->cexec = nullptr;
-        b->cgraph = nullptr;
-    }
-    b->bound = true;
-    return COLA_SUCCESS;
 }
 
 cola_status cola_batch_run(cola_batch *b, const cola_spmm_opts *opts, cola_stream_t stream)

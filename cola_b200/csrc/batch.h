@@ -66,6 +66,25 @@ inline dev::BlockArgs block_args(const cola_graph *g, float *ws, int64_t ld_ws)
     return ba;
 }
 
+// What one row-major product of a graph needs beside its operands: hub partials
+// (nseg rows of rows_ld_ws floats), room for the padded copy of X (rows_pad_bytes,
+// or NULL: X is read as it is), and dev::kMaxItemQueues + 1 work-item counters,
+// zero between products.  Products that share them must be ordered.
+struct RowsWork {
+    float *hub;
+    void *x_pad;
+    unsigned int *queue;
+};
+// Rows of the hub workspace are whole vectors of X.
+inline int64_t rows_ld_ws(cola_dtype xdt, int K)
+{
+    const int64_t E = xdt == COLA_FLOAT32 ? 4 : 8;
+    return (K + E - 1) / E * E;
+}
+size_t rows_pad_bytes(const cola_graph *g, cola_dtype xdt, const void *X, int64_t ldx, int K);
+cola_status rows_product(const cola_graph *g, const RowsWork &w, const void *X, cola_dtype xdt, int64_t ldx, void *Y,
+                         cola_dtype ydt, int64_t ldy, int K, const cola_spmm_opts *opts, cudaStream_t st);
+
 // Descriptor of graph g with these operands and hub workspace (item0 / hub0
 // left zero).
 void fill_batch_graph(dev::BatchGraph &d, const cola_graph *g, const void *X, int64_t ldx, void *Y, int64_t ldy,

@@ -561,42 +561,86 @@ bool vec_ok_rows(cola_dtype xdt, const void *X, int64_t ldx, cola_dtype ydt, con
     return true;
 }
 
-// X as the vector form reads it (a.xvec): itself where its rows are whole
-// aligned vectors, else a padded copy in the graph's workspace, else (few entries
-// a row, or no room on the device) left for the element-wise form, which gives
-// the same bits.  The copy is two passes over X, the element-wise form issues E
-// loads for one vector: padded from 16 entries a row on for FP32 X and 4 for BF16
-// (200 K rows, uniform, padded against element-wise in us: K = 33 FP32 at 4, 16,
-// 24 entries a row 54 / 44, 91 / 90, 113 / 118; K = 301 FP32 at 16 and 48 640 /
-// 606, 1460 / 1637; K = 33 BF16 at 2, 4, 16 39 / 34, 46 / 46, 77 / 104).
-static cola_status pad_x(cola_graph *g, RowsLaunch &a, bool capturing, cudaStream_t st)
+// Rows of X are whole aligned vectors.
+static bool vec_ok_x(cola_dtype xdt, const void *X, int64_t ldx, int K)
 {
-    const int E = a.xdt == COLA_FLOAT32 ? 4 : 8, esz = 16 / E;
-    a.xvec = a.K % E == 0 && a.ldx % E == 0 && a.ldx <= INT32_MAX / esz && aligned16(a.X);
-    if (a.xvec || g->nnz_l + g->nnz_r < (E == 4 ? 16 : 4) * (int64_t)g->NX)
-        return COLA_SUCCESS;
-    const int64_t nvec = (a.K + E - 1) / E;
-    const size_t bytes = (size_t)g->NX * nvec * 16;
-    if (grow(g->x_pad, bytes, capturing, g->kept) != COLA_SUCCESS) {
-        cudaGetLastError();
-        clear_error();
-        return COLA_SUCCESS;
-    }
-    const int64_t total = g->NX * nvec;
+    const int E = xdt == COLA_FLOAT32 ? 4 : 8;
+    return K % E == 0 && ldx % E == 0 && ldx <= INT32_MAX / (16 / E) && aligned16(X);
+}
+
+// X as the vector form reads it: itself where its rows are whole aligned
+// vectors, else a copy with padded rows, else (few entries a row, or no room on
+// the device) read by the element-wise form, which gives the same bits.  The copy
+// is two passes over X, the element-wise form issues E loads for one vector:
+// padded from 16 entries a row on for FP32 X and 4 for BF16 (200 K rows, uniform,
+// padded against element-wise in us: K = 33 FP32 at 4, 16, 24 entries a row 54 /
+// 44, 91 / 90, 113 / 118; K = 301 FP32 at 16 and 48 640 / 606, 1460 / 1637; K = 33
+// BF16 at 2, 4, 16 39 / 34, 46 / 46, 77 / 104).  Returns the copy's bytes, 0: none.
+size_t rows_pad_bytes(const cola_graph *g, cola_dtype xdt, const void *X, int64_t ldx, int K)
+{
+    const int E = xdt == COLA_FLOAT32 ? 4 : 8;
+    if (vec_ok_x(xdt, X, ldx, K) || g->nnz_l + g->nnz_r < (E == 4 ? 16 : 4) * (int64_t)g->NX)
+        return 0;
+    return (size_t)g->NX * ((K + E - 1) / E) * 16;
+}
+
+// Copies X to `pad` with padded rows; X and ldx become the copy's.
+static cola_status pad_x(const cola_graph *g, RowsLaunch &a, void *pad, cudaStream_t st)
+{
+    const int E = a.xdt == COLA_FLOAT32 ? 4 : 8;
+    const int64_t nvec = (a.K + E - 1) / E, total = g->NX * nvec;
     const unsigned blocks = (unsigned)std::min<int64_t>((total + dev::kThreads - 1) / dev::kThreads,
                                                         (int64_t)sm_count() * 32);
     t_launches++;
     if (a.xdt == COLA_FLOAT32)
         dev::pad_rows_kernel<float><<<blocks, dev::kThreads, 0, st>>>(
-            static_cast<const float *>(a.X), a.ldx, g->x_pad.f(), (int)nvec, total, a.K);
+            static_cast<const float *>(a.X), a.ldx, static_cast<float *>(pad), (int)nvec, total, a.K);
     else
         dev::pad_rows_kernel<__nv_bfloat16><<<blocks, dev::kThreads, 0, st>>>(
-            static_cast<const __nv_bfloat16 *>(a.X), a.ldx, static_cast<__nv_bfloat16 *>(g->x_pad.p), (int)nvec, total,
-            a.K);
+            static_cast<const __nv_bfloat16 *>(a.X), a.ldx, static_cast<__nv_bfloat16 *>(pad), (int)nvec, total, a.K);
     COLA_CUDA(cudaGetLastError());
-    a.X = g->x_pad.p;
+    a.X = pad;
     a.ldx = nvec * E;
-    a.xvec = true;
+    return COLA_SUCCESS;
+}
+
+cola_status rows_product(const cola_graph *g, const RowsWork &w, const void *X, cola_dtype xdt, int64_t ldx, void *Y,
+                         cola_dtype ydt, int64_t ldy, int K, const cola_spmm_opts *opts, cudaStream_t st)
+{
+    RowsLaunch a;
+    a.X = X;
+    a.ldx = ldx;
+    a.Y = Y;
+    a.ldy = ldy;
+    a.K = K;
+    a.xdt = xdt;
+    a.ydt = ydt;
+    a.vec = vec_ok_rows(xdt, X, ldx, ydt, Y, ldy, K);
+    a.accumulate = opts ? opts->accumulate : 0;
+    a.unroll = opts ? opts->unroll : 0;
+    a.min_blocks = opts ? opts->min_blocks : 0;
+    a.k_tile = opts ? opts->k_tile : 0;
+    if (w.x_pad)
+        COLA_TRY(pad_x(g, a, w.x_pad, st));
+    a.xvec = vec_ok_x(xdt, a.X, a.ldx, (w.x_pad ? (int)a.ldx : K));
+    const int64_t ldw = rows_ld_ws(xdt, K);
+    dev::BlockArgs ba = block_args(g, w.hub, ldw);
+    ba.queue = w.queue;
+    COLA_TRY(a.vec ? launch_block(ba, a, st) : launch_block_odd(ba, a, st));
+    if (g->nhub > 0) {
+        const unsigned blocks = hub_blocks(g->nhub * dev::hub_tiles(K), dev::hub_lanes(K));
+        t_launches++;
+        using BF = __nv_bfloat16;
+        if (ydt == COLA_FLOAT32) {
+            auto fn = a.vec ? dev::hub_combine_vec_kernel<float, true> : dev::hub_combine_vec_kernel<float, false>;
+            COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, w.hub, ldw,
+                                    static_cast<float *>(Y), ldy, K, a.accumulate));
+        } else {
+            auto fn = a.vec ? dev::hub_combine_vec_kernel<BF, true> : dev::hub_combine_vec_kernel<BF, false>;
+            COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, w.hub, ldw,
+                                    static_cast<BF *>(Y), ldy, K, a.accumulate));
+        }
+    }
     return COLA_SUCCESS;
 }
 
@@ -1303,43 +1347,16 @@ static cola_status spmm_impl(cola_graph *g, const void *X, cola_dtype xdt, int64
 
     if (schedule == COLA_SCHEDULE_ROWS) {
         // one writer per output row: Y written directly in its own dtype
-        // rows of the hub workspace are whole vectors of X
-        const int64_t E = xdt == COLA_FLOAT32 ? 4 : 8, ldw = (K + E - 1) / E * E;
         if (g->nseg > 0)
-            COLA_TRY(grow(g->ws_hub, (size_t)g->nseg * ldw * sizeof(float), capturing, g->kept));
-        RowsLaunch a;
-        a.X = X;
-        a.ldx = ldx;
-        a.Y = Y;
-        a.ldy = ldy;
-        a.K = K;
-        a.xdt = xdt;
-        a.ydt = ydt;
-        a.vec = vec_ok_rows(xdt, X, ldx, ydt, Y, ldy, K);
-        a.accumulate = accumulate;
-        a.unroll = opts ? opts->unroll : 0;
-        a.min_blocks = opts ? opts->min_blocks : 0;
-        a.k_tile = opts ? opts->k_tile : 0;
-        a.xvec = a.vec;
-        if (!a.vec)
-            COLA_TRY(pad_x(g, a, capturing, st));
-        const dev::BlockArgs ba = block_args(g, g->ws_hub.f(), ldw);
-        COLA_TRY(a.vec ? launch_block(ba, a, st) : launch_block_odd(ba, a, st));
-        if (g->nhub > 0) {
-            const unsigned blocks = hub_blocks(g->nhub * dev::hub_tiles(K), dev::hub_lanes(K));
-            t_launches++;
-            using BF = __nv_bfloat16;
-            if (ydt == COLA_FLOAT32) {
-                auto fn = a.vec ? dev::hub_combine_vec_kernel<float, true> : dev::hub_combine_vec_kernel<float, false>;
-                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw,
-                                        static_cast<float *>(Y), ldy, K, accumulate));
-            } else {
-                auto fn = a.vec ? dev::hub_combine_vec_kernel<BF, true> : dev::hub_combine_vec_kernel<BF, false>;
-                COLA_CUDA(launch_kernel(fn, blocks, 1, true, st, g->hub_row, g->hub_seg, g->nhub, g->ws_hub.f(), ldw,
-                                        static_cast<BF *>(Y), ldy, K, accumulate));
-            }
+            COLA_TRY(grow(g->ws_hub, (size_t)g->nseg * rows_ld_ws(xdt, K) * sizeof(float), capturing, g->kept));
+        size_t pad = rows_pad_bytes(g, xdt, X, ldx, K);
+        if (pad && grow(g->x_pad, pad, capturing, g->kept) != COLA_SUCCESS) {
+            cudaGetLastError();
+            clear_error();
+            pad = 0;
         }
-        return COLA_SUCCESS;
+        const RowsWork w{g->ws_hub.f(), pad ? g->x_pad.p : nullptr, g->item_queue};
+        return rows_product(g, w, X, xdt, ldx, Y, ydt, ldy, K, opts, st);
     }
 
     // accumulation target

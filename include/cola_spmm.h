@@ -530,16 +530,20 @@ cola_status cola_batch_create(const cola_partition_set *const *parts, int32_t ng
                               cola_batch **out, cola_stream_t stream);
 /* A batch over graphs that already exist (cola_graph_upload with the row
  * view, or cola_graph_build_device).  The batch borrows them (free the batch
- * first, then the graphs) and keeps a hub workspace of its own. */
+ * first, then the graphs) and keeps workspaces and work-item counters of its
+ * own, whatever the widths: other calls on the graphs need no ordering with
+ * the batch's, only runs of one batch among themselves. */
 cola_status cola_batch_create_from_graphs(cola_graph *const *graphs, int32_t ngraphs, cola_batch **out);
 cola_status cola_batch_free(cola_batch *b);
 
 /* Bind graph g's dense operands: X[g] (>= N_g rows, ldx[g]), Y[g] (N_g rows,
  * ldy[g]), width K[g]; every X in x_dtype, every Y in y_dtype.  Sizes the
  * workspaces and uploads the launch descriptors (synchronises `stream`); call
- * it again when a pointer changes.  Graphs whose operands are not 16-byte
- * vectors (K not a multiple of 4 FP32 / 8 BF16, unaligned rows) run through
- * cola_spmm inside cola_batch_run instead of the batched launch. */
+ * it again when a pointer changes (a caller's own capture of cola_batch_run
+ * refers to the binding it was made with: capture again after a bind).  Graphs
+ * whose operands are not 16-byte vectors (K not a multiple of 4 FP32 / 8 BF16,
+ * unaligned rows) run in launches of their own, as cola_spmm's, inside
+ * cola_batch_run instead of the batched launch. */
 cola_status cola_batch_bind(cola_batch *b, const void *const *X, const int64_t *ldx, void *const *Y,
                             const int64_t *ldy, const int32_t *K, cola_dtype x_dtype, cola_dtype y_dtype,
                             cola_stream_t stream);
