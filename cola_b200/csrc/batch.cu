@@ -474,7 +474,7 @@ cola_status cola_batch_get_info(const cola_batch *b, cola_batch_info *o)
     o->hub_items = b->total_hub;
     for (const cola_graph *g : b->graphs) {
         o->nnz += g->nnz_l + g->nnz_r;
-        o->device_bytes += (int64_t)(g->dbytes + g->ws_hub.bytes);
+        o->device_bytes += graph_bytes(g);
     }
     o->device_bytes += (int64_t)(b->d_desc_bytes + b->d_ws_bytes);
     o->unroll = b->unroll;

@@ -165,6 +165,12 @@ struct cola_graph {
 
 namespace cola {
 void graph_release(cola_graph *g);
+// Device memory a graph holds: its arrays and workspaces.
+inline int64_t graph_bytes(const cola_graph *g)
+{
+    return (int64_t)(g->dbytes + g->ppl_buf.bytes + g->stage_buf.bytes + g->ws.bytes + g->ws_hub.bytes +
+                     g->x_pad.bytes + g->kept.bytes());
+}
 
 // Row view parameters: the caller's cola_upload_opts fields where non-zero,
 // else chosen by the graph's size: with W warps in a full wave (32 per SM),

@@ -1250,8 +1250,7 @@ cola_status cola_graph_get_info(const cola_graph *g, cola_graph_info *o)
     o->local_chunks = g->lchunks;
     o->remote_chunks = g->rchunks;
     o->remote_cols = g->rcols;
-    o->device_bytes = (int64_t)(g->dbytes + g->ppl_buf.bytes + g->stage_buf.bytes + g->ws.bytes + g->ws_hub.bytes +
-                                  g->x_pad.bytes + g->kept.bytes());
+    o->device_bytes = graph_bytes(g);
     o->hub_rows = g->nhub;
     o->hub_segments = g->nseg;
     o->row_tasks = g->ntask;

@@ -276,7 +276,7 @@ cola_status cola_zip_rows_get_info(const cola_zip_rows *h, int64_t *rows, int64_
     if (hub_rows)
         *hub_rows = h->g->nhub;
     if (device_bytes)
-        *device_bytes = (int64_t)(h->g->dbytes + h->g->ws_hub.bytes);
+        *device_bytes = graph_bytes(h->g);
     return COLA_SUCCESS;
 }
 
