@@ -111,7 +111,8 @@ void host_pipe_release(HostPipe *p);
 
 struct cola_graph {
     int device = 0;
-    int32_t N = 0, NX = 0;  // rows of Y, rows of X (columns of the matrix)
+    int32_t N = 0;
+    int32_t x_row0 = 0, NX = 0;  // rows [x_row0, x_row0 + NX) of X hold every one that an entry names
     int32_t P = 0, npp = 0, gs = 0, nstages = 1, if_split = 1;
     int64_t nnz_l = 0, nnz_r = 0, lchunks = 0, rchunks = 0, rcols = 0;
     void *dmem = nullptr;

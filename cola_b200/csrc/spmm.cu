@@ -584,22 +584,25 @@ size_t rows_pad_bytes(const cola_graph *g, cola_dtype xdt, const void *X, int64_
     return (size_t)g->NX * ((K + E - 1) / E) * 16;
 }
 
-// Copies X to `pad` with padded rows; X and ldx become the copy's.
+// Copies X to `pad` with padded rows; X and ldx become the copy's.  Rows before
+// x_row0 are neither read nor there: the caller need not have them.
 static cola_status pad_x(const cola_graph *g, RowsLaunch &a, void *pad, cudaStream_t st)
 {
     const int E = a.xdt == COLA_FLOAT32 ? 4 : 8;
     const int64_t nvec = (a.K + E - 1) / E, total = g->NX * nvec;
     const unsigned blocks = (unsigned)std::min<int64_t>((total + dev::kThreads - 1) / dev::kThreads,
                                                         (int64_t)sm_count() * 32);
+    const int64_t first = g->x_row0 * a.ldx;
     t_launches++;
     if (a.xdt == COLA_FLOAT32)
         dev::pad_rows_kernel<float><<<blocks, dev::kThreads, 0, st>>>(
-            static_cast<const float *>(a.X), a.ldx, static_cast<float *>(pad), (int)nvec, total, a.K);
+            static_cast<const float *>(a.X) + first, a.ldx, static_cast<float *>(pad), (int)nvec, total, a.K);
     else
         dev::pad_rows_kernel<__nv_bfloat16><<<blocks, dev::kThreads, 0, st>>>(
-            static_cast<const __nv_bfloat16 *>(a.X), a.ldx, static_cast<__nv_bfloat16 *>(pad), (int)nvec, total, a.K);
+            static_cast<const __nv_bfloat16 *>(a.X) + first, a.ldx, static_cast<__nv_bfloat16 *>(pad), (int)nvec,
+            total, a.K);
     COLA_CUDA(cudaGetLastError());
-    a.X = pad;
+    a.X = static_cast<const char *>(pad) - g->x_row0 * nvec * 16;
     a.ldx = nvec * E;
     return COLA_SUCCESS;
 }

@@ -38,9 +38,10 @@ __global__ void expand_chunks_kernel(const int32_t *__restrict__ ptr, const int3
                                      int remote,
                                      int32_t *__restrict__ out_row, int32_t *__restrict__ out_col,
                                      float *__restrict__ out_val, unsigned int *__restrict__ max_row,
-                                     unsigned int *__restrict__ max_col, unsigned int *__restrict__ ok)
+                                     unsigned int *__restrict__ max_col, unsigned int *__restrict__ ok,
+                                     unsigned int *__restrict__ min_col)
 {
-    unsigned int mr = 0, mc = 0;
+    unsigned int mr = 0, mc = 0, lc = UINT32_MAX;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t e = e0 + i;
         // the chunk holding entry e: the last c with ptr[c] <= e
@@ -66,9 +67,11 @@ __global__ void expand_chunks_kernel(const int32_t *__restrict__ ptr, const int3
         out_val[i] = val ? __ldg(val + e) : 1.0f;
         mr = max(mr, (unsigned int)r);
         mc = max(mc, (unsigned int)c);
+        lc = min(lc, (unsigned int)c);
     }
     atomicMax(max_row, mr);
     atomicMax(max_col, mc);
+    atomicMin(min_col, lc);
 }
 
 static int blocks_for(int64_t n)
@@ -136,11 +139,11 @@ static cola_status build(const cola_zip_part *parts, int32_t nparts, const int64
     int32_t *row = reinterpret_cast<int32_t *>(base);
     int32_t *col = reinterpret_cast<int32_t *>(base + slice);
     float *val = reinterpret_cast<float *>(base + 2 * slice);
-    unsigned int *mx = reinterpret_cast<unsigned int *>(base + 3 * slice);  // max row, max col, all in range
+    unsigned int *mx = reinterpret_cast<unsigned int *>(base + 3 * slice);  // max row, max col, all in range, min col
     cola_status rc = COLA_SUCCESS;
-    unsigned int h_mx[3] = {0, 0, 1};
+    unsigned int h_mx[4] = {0, 0, 1, 0};
     {
-        const unsigned int init[3] = {0u, 0u, 1u};
+        const unsigned int init[4] = {0u, 0u, 1u, UINT32_MAX};
         cudaError_t e = cudaMemcpyAsync(mx, init, sizeof init, cudaMemcpyHostToDevice, st);
         int64_t at = 0;
         for (int32_t i = 0; i < nparts && e == cudaSuccess; i++) {
@@ -151,14 +154,15 @@ static cola_status build(const cola_zip_part *parts, int32_t nparts, const int64
                 expand_chunks_kernel<<<blocks_for(nl), 256, 0, st>>>(
                     z.csr_rowPtr_l, z.csr_rowIdx_zip_l, z.csr_colIdx_l, z.csr_val_l, z.local_row_lb, z.local_row_num,
                     en[0], nl, (int64_t)peids[i] * nodesPerPE, row0[i], 0, row + at, col + at, val + at, mx, mx + 1,
-                    mx + 2);
+                    mx + 2, mx + 3);
                 e = cudaGetLastError();
                 at += nl;
             }
             if (e == cudaSuccess && nr > 0) {
                 expand_chunks_kernel<<<blocks_for(nr), 256, 0, st>>>(
                     z.csc_colPtr_r, z.csc_colIdx_zip_r, z.csc_rowIdx_r, z.csc_val_r, z.remote_col_lb,
-                    z.remote_col_num, en[2], nr, 0, row0[i], 1, row + at, col + at, val + at, mx, mx + 1, mx + 2);
+                    z.remote_col_num, en[2], nr, 0, row0[i], 1, row + at, col + at, val + at, mx, mx + 1, mx + 2,
+                    mx + 3);
                 e = cudaGetLastError();
                 at += nr;
             }
@@ -179,6 +183,12 @@ static cola_status build(const cola_zip_part *parts, int32_t nparts, const int64
         const int64_t nrows = nnz > 0 ? (int64_t)h_mx[0] + 1 : 0;
         const int64_t ncols = std::max<int64_t>(nrows, nnz > 0 ? (int64_t)h_mx[1] + 1 : 0);
         rc = graph_build_device_rect((int32_t)nrows, (int32_t)ncols, nnz, row, col, val, nullptr, st, g, who);
+        // a caller need not have the rows of X before the first that an entry
+        // names, or past the last
+        if (rc == COLA_SUCCESS && nnz > 0) {
+            g->x_row0 = (int32_t)h_mx[3];
+            g->NX = (int32_t)(h_mx[1] - h_mx[3] + 1);
+        }
     }
     scratch_free(arena, 3 * slice + a, st);
     if (rc != COLA_SUCCESS)
