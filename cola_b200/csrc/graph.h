@@ -63,6 +63,9 @@ inline unsigned hub_blocks(int64_t items, int lanes)
     const int64_t per = dev::kThreads / lanes, need = (items + per - 1) / per, most = (int64_t)sm_count() * 16;
     return (unsigned)(need < 1 ? 1 : need < most ? need : most);
 }
+// Unique id of the calling thread's current CUDA context; 0 if there is none or
+// it cannot be read.
+unsigned long long current_context_id();
 // Device memory (memory.cu).  device_alloc: usable on every stream when it
 // returns; device_free: waits for the device first; both may be called while a
 // stream is being captured, by this thread or another.  scratch_alloc and

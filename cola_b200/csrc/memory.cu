@@ -25,21 +25,30 @@ struct DevicePool {
     cudaStream_t stream = nullptr;  // allocations that outlive a call are made on it
     void *anchor = nullptr;         // keeps the driver's chunk of small blocks, see wait_device
     bool tried = false;
+    unsigned long long context = 0;  // the context they belong to
 };
 
 static std::mutex g_pool_mu;
 static DevicePool g_pools[kMaxDevices];
 
-// The current device's pool; its members are NULL where it cannot be had.
+// The current device's pool; its members are NULL where it cannot be had.  One
+// that went with its context (cudaDeviceReset) is not used again.
 static DevicePool device_pool_entry()
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
         return DevicePool();
+    unsigned long long context = current_context_id();
+    if (context == 0) {
+        cudaFree(nullptr);  // makes the device's context
+        context = current_context_id();
+    }
     std::lock_guard<std::mutex> lk(g_pool_mu);
     DevicePool &p = g_pools[dev];
-    if (!p.tried) {
+    if (!p.tried || p.context != context) {
+        p = DevicePool();
         p.tried = true;
+        p.context = context;
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.handleTypes = cudaMemHandleTypeNone;

@@ -1495,10 +1495,9 @@ static __device__ __align__(256) float g_noalloc_stage[COLA_NOALLOC_STAGE_FLOATS
 
 namespace cola {
 
-// Unique id of the calling thread's current CUDA context (cuCtxGetId, reached
-// through the runtime's driver entry points, so the library does not link the
-// driver library itself); 0 if it cannot be read.
-static unsigned long long current_context_id()
+// cuCtxGetId, reached through the runtime's driver entry points, so the library
+// does not link the driver library itself.
+unsigned long long current_context_id()
 {
     using GetCurrent = CUresult (*)(CUcontext *);
     using GetId = CUresult (*)(CUcontext, unsigned long long *);
