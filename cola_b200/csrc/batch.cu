@@ -199,6 +199,10 @@ static cola_status batch_run(cola_batch *b, const cola_spmm_opts *opts, cudaStre
     const int accumulate = opts ? opts->accumulate : 0;
     COLA_REQUIRE(!(accumulate && b->ydt != COLA_FLOAT32), COLA_ERROR_UNSUPPORTED,
                  "cola_batch_run: accumulate needs FP32 outputs");
+    int cur = 0;
+    COLA_CUDA(cudaGetDevice(&cur));
+    COLA_REQUIRE(cur == b->device, COLA_ERROR_INVALID_ARGUMENT,
+                 "cola_batch_run: batch lives on device %d, current device is %d", b->device, cur);
     const int64_t before = t_launches;
     BatchLaunch L = b->launch;
     L.desc = b->d_desc;

@@ -40,6 +40,8 @@ std::vector<Cand> rows_candidates(cola_dtype xdt, int K)
     for (int kt : tiles) {
         if (xdt == COLA_FLOAT32 && kt == 1024)
             continue;
+        if (kt > 64 * e16 && kt < K)  // swept 64 vectors at a time, the candidate before it
+            continue;
         if (kt > 64 && kt / 2 >= K)  // wider than K needs
             continue;
         const bool narrow = kt * (xdt == COLA_FLOAT32 ? 4 : 2) < 512;

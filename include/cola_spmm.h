@@ -460,12 +460,14 @@ typedef struct cola_spmm_opts {
     int32_t schedule;           /* enum cola_schedule */
     int32_t gather_batch_rows;  /* staging batch (rows) for BUFFER/PIPELINE; 0 = 4096 */
     int32_t unroll;             /* ROWS: row loads in flight per lane group (2, 4, 6 or 8; 6 runs as 8; 0 = 4) */
-    int32_t min_blocks;         /* ROWS: resident blocks per SM the kernel is compiled for (3, 4, 5, 6;
-                                   0 = 3 for FP32 X, 4 for BF16 X) */
+    int32_t min_blocks;         /* ROWS, K of one vector a lane (128 FP32 X, 256 BF16 X): resident blocks per SM
+                                   the kernel is compiled for (3, 4, 5, 6; 0 = 4); wider K runs at 3, or 4
+                                   with unroll 2 */
     int32_t k_tile;             /* ROWS, K >= 128 (FP32 X) or >= 256 (BF16 X): features per pass over the
                                    graph (64, 128, 256, 512, 1024; 0 = chosen by the library).  The passes
-                                   run one after another so the X columns in use are one tile wide; every
-                                   choice gives the same bits.  Ignored for narrower K. */
+                                   run one after another so the X columns in use are one tile wide; a pass
+                                   of a K wider than k_tile is at most 256 (FP32 X) or 512 (BF16 X)
+                                   features.  Every choice gives the same bits.  Ignored for narrower K. */
     int32_t reserved[2];
 } cola_spmm_opts;
 
