@@ -12,11 +12,18 @@ from .prep import (PartitionSet, bin2vec, community_order, global_csr, nnz_split
 
 __all__ = ["PartitionSet", "row_partition", "serialize", "ppl_row_partition", "nnz_split", "nnz_split_device",
            "relabel_edges", "community_order", "stage_tables",
-           "workgroup_cols", "global_csr", "bin2vec", "write_bin", "rmat", "ColaError", "lib", "version"]
+           "workgroup_cols", "global_csr", "bin2vec", "write_bin", "rmat", "ColaError", "lib", "trim_memory", "version"]
 
 
 def version():
     return _lib.lib().cola_version().decode()
+
+
+def trim_memory():
+    """Give the device memory the library keeps for reuse (up to 1 GiB a device,
+    freed by earlier builds and graphs) back to the device, for other allocators
+    of the process; waits for the current device."""
+    _lib.check(_lib.lib().cola_trim_memory())
 
 
 def __getattr__(name):

@@ -22,7 +22,7 @@ def edges(n, m, seed):
 @pytest.mark.parametrize("mode,thread", [("thread_local", True), ("relaxed", True), ("global", True),
                                          ("thread_local", False), ("global", False)])
 def test_free_during_a_capture(mode, thread):
-    n, m = 50000, 1 << 20
+    n, m = 50000, 1 << 24
     coo = edges(n, m, 1)
     g = S.Graph.from_coo_device(n, *coo)
     x = torch.randn((n, 32), device=DEV)
@@ -49,7 +49,9 @@ def test_free_during_a_capture(mode, thread):
     torch.cuda.synchronize()
     assert torch.equal(b, 2 * a + 1)
     assert cb.lib().cola_trim_memory() == 0
-    assert torch.cuda.mem_get_info()[0] - before >= m * 8  # the graph's columns and values at least
+    # the graph's columns and values at least; chunks at its ends may be shared with
+    # graphs that are alive
+    assert torch.cuda.mem_get_info()[0] - before >= m * 8 - (64 << 20) > 0
 
 
 def test_free_waits_for_running_products():
