@@ -1,13 +1,13 @@
 // Device memory of the library: one stream-ordered pool per device that keeps
 // up to kKeep bytes mapped after they are freed.  Mapping and unmapping cost
 // about 7 ms a gigabyte each with the default pool (which unmaps at every
-// synchronisation) and 0.5 ms or more per cudaMalloc or cudaFree, most of the
-// wall time of building a graph (1 M rows, 14 M entries, and one SpMM: 4.8 ms and
-// up to 29 on a busy host, 1.8 with the pool).  The kept bytes are given back by
-// cola_trim_memory and before the library reports that the device is full; the
-// driver gives back what exceeds kKeep at each synchronisation.  Pools are safe
-// with several threads and streams: memory freed on one stream is handed to
-// another only in order.
+// synchronisation) and 0.3 to 0.6 ms per cudaMalloc or cudaFree of 16 to 480 MB,
+// most of the wall time of building a graph (1 M rows, 14 M entries, and one
+// SpMM: 4.8 ms and up to 29 on a busy host, 1.7 with the pool).  The kept bytes
+// are given back by cola_trim_memory and before the library reports that the
+// device is full; the driver gives back what exceeds kKeep at each
+// synchronisation.  Pools are safe with several threads and streams: memory freed
+// on one stream is handed to another only in order.
 #include <mutex>
 
 #include <cuda_runtime.h>

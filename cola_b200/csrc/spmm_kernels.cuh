@@ -168,6 +168,9 @@ struct ScalarTraits {
 // ends inside a vector): as many features a lane as VecTraits, but LG apart, so
 // that neighbouring lanes read neighbouring elements.  A feature is summed by
 // the same lane group in the same order as in the vector form: the same bits.
+// Bound by the loads it issues, E for one vector, where rows are long, and by the
+// gathers' latency where they are short (200 K rows, 1.5 entries a row, against a
+// scalar kernel of one warp a row: K = 33 FP32 50 -> 28 us, K = 301 BF16 167 -> 83).
 template <typename T>
 struct LooseTraits {
     static constexpr int E = 16 / (int)sizeof(T);

@@ -204,15 +204,17 @@ __device__ __forceinline__ unsigned int warp_in_block()
 // What bounds it: the L1/L2 gather traffic of X with UNROLL x resident warps
 // rows in flight; instruction issue comes next, so a round inside one row costs
 // 3 shared loads, one address and one load per entry, and the products.
-// Measured (R-MAT, one lane group a row): scale 20, K = 128 FP32 1.11 -> 1.07 ms
-// against the form that walked row pointers, scale 21, K = 256 BF16 4.03 ->
-// 3.85, uniform rows of 20 entries at K = 100 83 -> 74 us; narrow rows: K = 16
-// BF16 206 -> 117 us, K = 32 FP32 on 16 K rows 23 -> 13 us.  Slower: 8 rows in
+// Measured against the form that walked row pointers (R-MAT, one lane group a
+// row, one product under ncu): scale 20, K = 128 FP32 1.084 -> 1.042 ms, scale 21,
+// K = 256 BF16 3.94 -> 3.86; uniform rows of 20 entries at K = 100 83 -> 74 us;
+// narrow rows: K = 16 BF16 206 -> 117 us, K = 32 FP32 on 16 K rows 23 -> 13 us.
+// Slower (scale 20, K = 128 FP32, 1.07 ms in the same runs): 8 rows in
 // flight at 3 blocks (1.10 ms), 2 at 5 or 6 (1.35), the next row's load issued
 // as each row is added (1.64).
 // VEC_Y: rows of Y are written in vectors; else (their start is not aligned or K
-// ends inside a vector of X) element by element, X still read in vectors.  RED:
-// sums are added to Y with reductions (other warps add to the same rows).
+// ends inside a vector of X) element by element, X read in vectors or, with
+// LooseTraits, element by element too.  RED: sums are added to Y with reductions
+// (other warps add to the same rows).
 template <typename TR, typename TY, int LG, int NV, int UNROLL, bool VEC_Y = true, bool RED = false>
 struct RowStream {
     using T = typename ElemOf<TR>::T;

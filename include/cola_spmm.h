@@ -307,8 +307,9 @@ typedef struct cola_zip_part {
 cola_status cola_zip_rows_create_all(const cola_zip_part *parts, int32_t nparts, int32_t nodesPerPE,
                                      cola_stream_t stream, cola_zip_rows **out);
 /* output[r] += sum of the covered entries of row r times input rows (input =
- * PE peid's slice of the symmetric X, as for cola_ppl0_batch_spmm); FP32,
- * any dim >= 1.  Asynchronous on `stream`. */
+ * PE peid's slice of the symmetric X, as for cola_ppl0_batch_spmm; only rows
+ * from the first to the last that an entry names are read); FP32, any dim >= 1.
+ * Asynchronous on `stream`. */
 cola_status cola_zip_rows_spmm(cola_zip_rows *h, float *output, const float *input, int32_t dim,
                                cola_stream_t stream);
 cola_status cola_zip_rows_free(cola_zip_rows *h);
@@ -477,9 +478,11 @@ typedef struct cola_spmm_opts {
  * widened exactly and accumulated in FP32); y_dtype FP32 or BF16 (rounded
  * once, at the end).  opts may be NULL.  The ROWS schedule hands its work
  * items (hub segments, row blocks) to warps from counters kept in the graph,
- * and hub rows' partial sums go to a workspace of the graph: calls on one
- * graph that overlap on the GPU (different streams or threads) race on both
- * and must be serialised by the caller; calls on one stream are. */
+ * and hub rows' partial sums and, at widths and alignments no 16-byte vector
+ * divides, a copy of X with padded rows go to workspaces of the graph: calls on
+ * one graph that overlap on the GPU (different streams or threads) race on them
+ * and must be serialised by the caller; calls on one stream are.  A captured
+ * call keeps the workspaces it was captured with until the graph is freed. */
 cola_status cola_spmm(cola_graph *g, const void *X, cola_dtype x_dtype, int64_t ldx, void *Y, cola_dtype y_dtype,
                       int64_t ldy, int32_t K, const cola_spmm_opts *opts, cola_stream_t stream);
 
